@@ -13,6 +13,8 @@ constexpr int kMaxFilmLayers = 8;  // thin-film layers handled by the FP32 trans
 struct DeviceScene {
     const float4 *nodes;         // binary BVH (min, index) (max, count): root boxes
     const float4 *wide;          // wide BVH child records, `width` per node (wide_bvh.h)
+    const float *wide_planes;    // the same boxes and codes by plane (child_boxes): per node `width` floats each of
+                                 // min x, max x, min y, max y, min z, max z, the codes, and padding
     const int2 *wide_leaves;     // (index, count) of every binary leaf
     const int *wide_code;        // per binary node: wide code of the tree roots
     const uint4 *wide_q;         // compressed node records (wide_bvh.h), kQuantWords per node

@@ -320,6 +320,7 @@ DeviceScene lambda_ctx::scene_view(int width) const {
     const int k = width == 2 ? 0 : (width == 4 ? 1 : 2);
     DeviceScene v = dscene;
     v.wide = scene.wide[k].as<float4>();
+    v.wide_planes = scene.wide_planes[k].as<float>();
     v.wide_leaves = scene.wide_leaves[k].as<int2>();
     v.wide_code = scene.wide_code[k].as<int>();
     v.wide_q = scene.wide_q[k].as<uint4>();
@@ -333,6 +334,22 @@ DeviceScene lambda_ctx::scene_view(int width) const {
     }
     return v;
 }
+
+namespace {
+
+// Child records (8 floats: min, code, max, 0) of every wide node to the plane form of
+// child_boxes: field f of child i at [node][f][i], fields min x, max x, min y, max y,
+// min z, max z, code, 0. One thread per output float.
+__global__ void k_wide_planes(const float *records, int width, size_t n, float *planes) {
+    const size_t k = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const size_t node = k / (8 * width);
+    const int r = int(k % (8 * width)), f = r / width, i = r % width;
+    const int src[8] = {0, 4, 1, 5, 2, 6, 3, 7};
+    planes[k] = records[(node * width + i) * 8 + src[f]];
+}
+
+}  // namespace
 
 extern "C" lambda_status lambda_scene_upload(lambda_ctx *ctx, const lambda_scene_desc *desc) {
     if (!ctx || !desc) return LAMBDA_ERR_INVALID_ARGUMENT;
@@ -497,6 +514,12 @@ extern "C" lambda_status lambda_scene_upload(lambda_ctx *ctx, const lambda_scene
         CK(b.wide_leaves[k].upload(w.leaves.data(), w.leaves.size() * sizeof(int32_t), s), "upload wide BVH");
         CK(b.wide_code[k].upload(w.code.data(), w.code.size() * sizeof(int32_t), s), "upload wide BVH");
         CK(b.wide_q[k].upload(w.quant.data(), w.quant.size() * sizeof(uint32_t), s), "upload wide BVH");
+        const size_t floats = w.records.size() / (size_t(16) << k) * (size_t(16) << k);  // whole nodes of 8 * width floats
+        CK(b.wide_planes[k].reserve(w.records.size() * sizeof(float)), "upload wide BVH");
+        if (floats > 0)
+            k_wide_planes<<<unsigned((floats + 255) / 256), 256, 0, s>>>(b.wide[k].as<float>(), 2 << k, floats,
+                                                                        b.wide_planes[k].as<float>());
+        CK(cudaGetLastError(), "upload wide BVH");
         ctx->wide_leaves_n[k] = int(w.leaves.size() / 2);
         CK(cudaStreamSynchronize(s), "upload wide BVH");  // the host vectors go out of scope
         ctx->wide_stack[k][0] = w.stack_tlas;

@@ -52,6 +52,7 @@ struct SceneBuffers {
         material_uv, film_flat,
         cie, perm, worley, instance_flags;
     DeviceBuffer wide[3], wide_leaves[3], wide_code[3];  // wide BVH of width 2, 4, 8
+    DeviceBuffer wide_planes[3];                          // the child boxes and codes by plane
     DeviceBuffer wide_q[3];                               // its compressed node records
 };
 
@@ -121,7 +122,7 @@ struct lambda_ctx {
                 &s.cspectrum_flat, &s.materials, &s.material_props, &s.scalar_tex, &s.spectrum_tex, &s.light_inst,
                 &s.light_obj, &s.light_power, &s.light_cdf, &s.material_emission, &s.material_uv, &s.film_flat, &s.cie, &s.perm, &s.worley, &s.instance_flags,
                 &s.wide[0], &s.wide[1], &s.wide[2], &s.wide_leaves[0], &s.wide_leaves[1], &s.wide_leaves[2],
-                &s.wide_code[0], &s.wide_code[1], &s.wide_code[2], &s.wide_q[0], &s.wide_q[1], &s.wide_q[2],
+                &s.wide_code[0], &s.wide_code[1], &s.wide_code[2], &s.wide_planes[0], &s.wide_planes[1], &s.wide_planes[2], &s.wide_q[0], &s.wide_q[1], &s.wide_q[2],
                 &r.rng, &r.film, &r.lam, &r.ray_o, &r.ray_d, &r.throughput, &r.radiance, &r.emit, &r.hit_id,
                 &r.sh_o, &r.sh_d, &r.sh_a, &r.sh_light, &r.q0, &r.q1, &r.qs, &r.qm0, &r.qm1, &r.qm2, &r.counts, &r.wave,
                 &r.stats, &r.error, &r.out, &r.path_info, &r.jobs, &r.active, &r.work, &r.film_rows, &r.film_out,
