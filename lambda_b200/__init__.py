@@ -430,7 +430,8 @@ def default_film_range() -> N.FilmRange:
 # structure-of-arrays words the stage must read and write (queue ids included),
 # not counting scene data, which is read-only and cache resident for small scenes.
 STAGE_BYTES = {
-    "raygen": 16 * 2 + 16 * 2 + 16 + 8 * 2 + 16 * 4 + 4,   # film rw, radiance rw, lam w, rng rw, ray/T w, queue
+    # film rw, radiance rw, lam rw, rng rw, hit id, ray/T w, queue (and the ray and T of a miss or an emitter hit)
+    "raygen": 16 * 2 + 16 * 2 + 16 * 2 + 8 * 2 + 16 + 16 * 3 + 4,
     "intersect": 4 + 32 + 16 + 4,                          # queue id, ray read, hit id write, material push
     # the shade kernels rebuild the hit record from the ray and the hit id
     "shade_lambert": 4 + 32 + 16 + 16 * 2 + 8 * 2 + 32 + 16 + 64 + 8,  # queue, ray, hit id, T/lam, rng rw, ray w, T w, NEE w, pushes

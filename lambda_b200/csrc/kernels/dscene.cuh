@@ -256,8 +256,11 @@ __device__ __forceinline__ s4 spectrum_texture4(const DeviceScene &s, int t, con
 __device__ __forceinline__ s4 background_eval(const DeviceScene &s, f3 d, const s4 &lam) {
     ShadePoint sp;
     sp.point = d;
-    sp.u = (atan2f(d.z, d.x) + kPi) / (2 * kPi);
-    sp.v = acosf(d.y) / kPi;
+    sp.u = sp.v = 0.0f;
+    if (__ldg(&s.spectrum_tex[s.background_texture].x) == 1) {  // only a checker reads (u, v)
+        sp.u = (atan2f(d.z, d.x) + kPi) / (2 * kPi);
+        sp.v = acosf(d.y) / kPi;
+    }
     return spectrum_texture4(s, s.background_texture, sp, lam);
 }
 
@@ -441,20 +444,27 @@ __device__ __forceinline__ void prim_attributes(const DeviceScene &s, int obj, c
     if (!h.front) h.normal = h.normal * -1.0f;
 }
 
-// Traversal stack of one thread in shared memory, entry-major (entry i of thread t
-// at base[i * stride + t], so a warp's pushes and pops hit 32 different banks). An
-// entry is a wide-BVH code and the entry distance of its box. The capacity is the
-// most entries the scene's trees can need (computed when the scene is uploaded).
-struct WideStack {
-    int *code;
-    float *te;
+// Traversal stack of one thread in shared memory, entry-major (entry i of thread t at
+// e[i * stride + t]). An entry is a wide-BVH code and the entry distance of its box.
+// The capacity is the most entries the scene's trees can need (computed when the
+// scene is uploaded). Every walk of a kernel keeps to its own thread's column of the
+// block's stack memory, so the threads of a block may run different walks at once.
+struct TravStack {
+    int2 *e;
     int stride;
     int cap;
-    __device__ __forceinline__ void put(int i, int c, float t) const {
-        code[i * stride] = c;
-        te[i * stride] = t;
+    __device__ __forceinline__ void put(int i, int c, float t) const { e[i * stride] = make_int2(c, __float_as_int(t)); }
+    __device__ __forceinline__ void get(int i, int &c, float &t) const {
+        const int2 v = e[i * stride];
+        c = v.x;
+        t = __int_as_float(v.y);
     }
 };
+
+// The TLAS stack a and the BLAS stack b after it (wide_stacks), as one stack.
+__device__ __forceinline__ TravStack trav_stack(const TravStack &a, const TravStack &b) {
+    return TravStack{a.e, a.stride, a.cap + b.cap};
+}
 
 // World ray wr -> instance space (instance.h:50-52), given the instance's flags. An
 // identity instance's transform reduces exactly to adding +0 (which only turns -0
@@ -620,7 +630,7 @@ __device__ __forceinline__ float qbyte(const uint32_t (&b)[N], int i) {
 // (one multiply, one add, as the encoder checked them), and each child that passes
 // is pushed as its record slot.
 template <int L>
-__device__ __forceinline__ int wide_expand(const DeviceScene &s, int w, const Ray3 &r, float best, const WideStack &st,
+__device__ __forceinline__ int wide_expand(const DeviceScene &s, int w, const Ray3 &r, float best, const TravStack &st,
                                            int sp, bool &overflow) {
     constexpr int K = kWidthOf<L>;
     const float4 *c = s.wide + size_t(w) * (2 * K);
@@ -728,8 +738,8 @@ __device__ __forceinline__ bool closest_hit_finish(const DeviceScene &s, const R
 // record from them.
 template <int K>
 __device__ __forceinline__ void closest_hit_ids_w(const DeviceScene &s, const Ray3 &wr, float &best, int &best_obj,
-                                                  int &best_inst, bool &overflow, const WideStack &st,
-                                                  const WideStack &sub) {
+                                                  int &best_inst, bool &overflow, const TravStack &st,
+                                                  const TravStack &sub) {
     best = kMax;
     best_obj = -1;
     best_inst = -1;
@@ -738,8 +748,9 @@ __device__ __forceinline__ void closest_hit_ids_w(const DeviceScene &s, const Ra
     if (slab(__ldg(&s.nodes[0]), __ldg(&s.nodes[1]), wr, te)) st.put(sp++, root_entry<K>(s, __ldg(&s.wide_code[0])), te);
     while (sp > 0) {
         --sp;
-        te = st.te[sp * st.stride];
-        const int code = pop_code<K>(s, st.code[sp * st.stride], te, wr, best);
+        int code;
+        st.get(sp, code, te);
+        code = pop_code<K>(s, code, te, wr, best);
         if (code == INT_MIN) continue;
         if (code >= 0) {
             sp = wide_expand<K>(s, code, wr, best, st, sp, overflow);
@@ -758,8 +769,10 @@ __device__ __forceinline__ void closest_hit_ids_w(const DeviceScene &s, const Ra
         sub.put(ssp++, root_entry<K>(s, __ldg(&s.wide_code[root])), te);
         while (ssp > 0) {
             --ssp;
-            float te2 = sub.te[ssp * sub.stride];
-            const int c2 = pop_code<K>(s, sub.code[ssp * sub.stride], te2, lr, best);
+            float te2;
+            int c2;
+            sub.get(ssp, c2, te2);
+            c2 = pop_code<K>(s, c2, te2, lr, best);
             if (c2 == INT_MIN) continue;
             if (c2 >= 0) {
                 ssp = wide_expand<K>(s, c2, lr, best, sub, ssp, overflow);
@@ -780,15 +793,114 @@ __device__ __forceinline__ void closest_hit_ids_w(const DeviceScene &s, const Ra
     }
 }
 
-// Scene::hit in closest-hit mode with the hit record. Returns false on a miss.
+// Expands wide node `code` over an exact layout: the passing child visited first becomes
+// the next node (`code`, `te`), the others are pushed, last-visited first. Returns
+// false when no child passes, or when the stack is full (`overflow`).
 template <int K>
-__device__ __forceinline__ bool closest_hit_w(const DeviceScene &s, f3 o, f3 d, Hit &h, bool &overflow,
-                                              const WideStack &st, const WideStack &sub) {
-    const Ray3 wr = make_ray(o, d);
-    float best;
-    int best_obj, best_inst;
-    closest_hit_ids_w<K>(s, wr, best, best_obj, best_inst, overflow, st, sub);
-    return closest_hit_finish(s, wr, best, best_obj, best_inst, h);
+__device__ __forceinline__ bool expand_next(const DeviceScene &s, const Ray3 &r, float best, const TravStack &st, int &sp,
+                                            int cap, int &code, float &te, bool &overflow) {
+    ChildBoxes<K> cb;
+    child_boxes<K>(s, code, r, best, cb);
+    bool pass[K], any = false;
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+        pass[i] = cb.te[i] <= cb.tf[i];
+        any = any || pass[i];
+    }
+    if (!any) return false;
+    if (sp + K > cap) {  // not room for every child: count the ones that passed
+        int n = 0;
+#pragma unroll
+        for (int i = 0; i < K; i++) n += pass[i] ? 1 : 0;
+        if (sp + n > cap) {
+            overflow = true;
+            return false;
+        }
+    }
+    bool have = false;
+#pragma unroll
+    for (int i = K - 1; i >= 0; i--) {
+        if (pass[i]) {
+            if (have) st.put(sp++, code, te);
+            code = cb.code[i];
+            te = cb.te[i];
+            have = true;
+        }
+    }
+    return true;
+}
+
+// One ray's closest-hit walk as closest_hit_ids_w makes it, one node per step(): the
+// same nodes in the same order against the same best distance. TLAS and BLAS share
+// the loop, the stack and the expansion code: `r` is the ray of the level being
+// walked, `base` the stack height at which the current BLAS began (-1 in the TLAS) and
+// `cap` the height its level may reach.
+struct FlatWalk {
+    Ray3 r;
+    float best, te;
+    int obj, hit_inst, inst, code, sp, base, cap;
+};
+
+// Starts the walk of world ray wr. Returns false when the ray misses the scene's box.
+__device__ __forceinline__ bool flat_start(const DeviceScene &s, const Ray3 &wr, FlatWalk &w) {
+    w.best = kMax;
+    w.obj = w.hit_inst = w.inst = -1;
+    w.sp = 0;
+    w.base = -1;
+    w.cap = s.stack_tlas;
+    w.r = wr;
+    w.code = __ldg(&s.wide_code[0]);
+    return slab(__ldg(&s.nodes[0]), __ldg(&s.nodes[1]), wr, w.te);
+}
+
+// Visits one node; returns false when the walk is done.
+template <int K>
+__device__ __forceinline__ bool flat_step(const DeviceScene &s, const Ray3 &wr, FlatWalk &w, const TravStack &st,
+                                          bool &overflow) {
+    if (w.code >= 0) {
+        if (expand_next<K>(s, w.r, w.best, st, w.sp, w.cap, w.code, w.te, overflow)) return true;
+        if (overflow) return false;
+    } else {
+        const int2 lf = __ldg(&s.wide_leaves[-w.code - 1]);
+        if (w.base >= 0) {
+            for (int k = 0; k < lf.y; k++) {
+                const float t = intersect_t(load_prim(s, lf.x + k), w.r, w.best);
+                if (t >= 0) {
+                    w.best = t;
+                    w.obj = lf.x + k;
+                    w.hit_inst = w.inst;
+                }
+            }
+        } else {
+            // a TLAS leaf: its first instance only (scene.h:80)
+            w.inst = lf.x;
+            const uint32_t flags = s.instance_flags[lf.x];
+            const InstanceRef ir = instance_ref(s, lf.x);
+            const int root = ir.header().z;
+            const Ray3 lr = to_local(flags, ir, wr);
+            float te = w.te;
+            if ((flags & 2u) ||
+                (slab(__ldg(&s.nodes[2 * root]), __ldg(&s.nodes[2 * root + 1]), lr, te) && !(te > w.best))) {
+                w.r = lr;
+                w.base = w.sp;
+                w.cap = w.sp + s.stack_blas;
+                w.te = te;
+                w.code = __ldg(&s.wide_code[root]);
+                return true;
+            }
+        }
+    }
+    for (;;) {
+        if (w.sp == w.base) {
+            w.base = -1;
+            w.cap = s.stack_tlas;
+            w.r = wr;
+        }
+        if (w.sp == 0) return false;
+        --w.sp;
+        st.get(w.sp, w.code, w.te);
+        if (!(w.te > w.best)) return true;
+    }
 }
 
 // Scene::hit in shadow mode (scene.h:51-124 with occludedInstance/Object) over the
@@ -798,7 +910,7 @@ __device__ __forceinline__ bool closest_hit_w(const DeviceScene &s, f3 o, f3 d, 
 // light, `light` holds the light's hit record for its emission lookup.
 template <int K>
 __device__ __forceinline__ bool occluded_w(const DeviceScene &s, f3 o, f3 d, int light_inst, int light_obj, Hit &light,
-                                           bool &overflow, const WideStack &st, const WideStack &sub) {
+                                           bool &overflow, const TravStack &st, const TravStack &sub) {
     const Ray3 wr = make_ray(o, d);
     float best = kMax;
     if (light_inst != -1) {
@@ -818,8 +930,9 @@ __device__ __forceinline__ bool occluded_w(const DeviceScene &s, f3 o, f3 d, int
     if (slab(__ldg(&s.nodes[0]), __ldg(&s.nodes[1]), wr, te)) st.put(sp++, root_entry<K>(s, __ldg(&s.wide_code[0])), te);
     while (sp > 0) {
         --sp;
-        te = st.te[sp * st.stride];
-        const int code = pop_code<K>(s, st.code[sp * st.stride], te, wr, best);
+        int code;
+        st.get(sp, code, te);
+        code = pop_code<K>(s, code, te, wr, best);
         if (code == INT_MIN) continue;
         if (code >= 0) {
             sp = wide_expand<K>(s, code, wr, best, st, sp, overflow);
@@ -837,8 +950,10 @@ __device__ __forceinline__ bool occluded_w(const DeviceScene &s, f3 o, f3 d, int
         sub.put(ssp++, root_entry<K>(s, __ldg(&s.wide_code[root])), te);
         while (ssp > 0) {
             --ssp;
-            float te2 = sub.te[ssp * sub.stride];
-            const int c2 = pop_code<K>(s, sub.code[ssp * sub.stride], te2, lr, best);
+            float te2;
+            int c2;
+            sub.get(ssp, c2, te2);
+            c2 = pop_code<K>(s, c2, te2, lr, best);
             if (c2 == INT_MIN) continue;
             if (c2 >= 0) {
                 ssp = wide_expand<K>(s, c2, lr, best, sub, ssp, overflow);
@@ -855,12 +970,13 @@ __device__ __forceinline__ bool occluded_w(const DeviceScene &s, f3 o, f3 d, int
     return false;
 }
 
-// The two traversal stacks of this thread in dynamic shared memory: TLAS codes,
-// TLAS distances, BLAS codes, BLAS distances, each [cap][blockDim.x].
-__device__ __forceinline__ void wide_stacks(int *smem, const DeviceScene &s, WideStack &a, WideStack &b) {
-    const int B = blockDim.x, t = threadIdx.x, ca = s.stack_tlas, cb = s.stack_blas;
-    a = WideStack{smem + t, reinterpret_cast<float *>(smem + ca * B) + t, B, ca};
-    b = WideStack{smem + 2 * ca * B + t, reinterpret_cast<float *>(smem + 2 * ca * B + cb * B) + t, B, cb};
+// The two traversal stacks of this thread in dynamic shared memory: the TLAS entries,
+// then the BLAS entries, each [cap][blockDim.x].
+__device__ __forceinline__ void wide_stacks(int *smem, const DeviceScene &s, TravStack &a, TravStack &b) {
+    const int B = blockDim.x, ca = s.stack_tlas, cb = s.stack_blas;
+    int2 *e = reinterpret_cast<int2 *>(smem) + threadIdx.x;
+    a = TravStack{e, B, ca};
+    b = TravStack{e + ca * B, B, cb};
 }
 
 __host__ __device__ inline size_t wide_stack_bytes(int block, int stack_tlas, int stack_blas) {

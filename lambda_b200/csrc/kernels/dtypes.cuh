@@ -80,6 +80,8 @@ struct RenderParams {
     const int2 *work;   // [num_jobs]
 };
 
+enum : int { kMissed = -1, kNoHit = -2 };  // PathState::hit_id objects
+
 struct PathState {
     uint64_t *rng;        // PCG32 state per pixel
     float4 *film;         // accumulated linear sRGB (xyz)
@@ -88,8 +90,8 @@ struct PathState {
     float4 *ray_d;        // direction xyz, w = 1 if the last scatter was specular
     float4 *throughput;
     float4 *radiance;     // NEE terms of the running sample
-    float4 *emit;         // emission term of a sample that ended at a miss or an emitter
-    int4 *hit_id;         // material, object, distance (float bits), instance of a stored hit
+    int4 *hit_id;         // material, object, distance (float bits), instance of the last closest hit;
+                          // object kMissed: it met nothing, kNoHit: no closest hit since the sample was banked
     float4 *sh_o;         // NEE ray origin xyz, w = MIS weight
     float4 *sh_d;         // NEE ray direction xyz, w = light pdf
     float4 *sh_a;         // throughput * BSDF * cos

@@ -4,19 +4,20 @@
 // consumed in the reference's order (renderer.h:64-92, :94-195), so each pixel
 // must finish sample s before it starts s+1, and the wave is the unit of
 // parallelism (W*H paths in flight). Per bounce i the stages are
-//   intersect   closest hit of every active path (scene.h:51); misses and emitter
-//               hits are finished on the spot (renderer.h:105-131), the rest are
-//               pushed to one queue per material family
+//   intersect   closest hit of every active path (scene.h:51); a miss or an emitter
+//               hit ends the path (renderer.h:105-131), the rest are pushed to one
+//               queue per material family
 //   lambert     NEE light sampling + cosine scatter + Russian roulette (renderer.h:133-191)
 //   specular    mirror and dielectric scatter + Russian roulette
 //   thin film   transfer-matrix reflectance of the four hero wavelengths, scatter
 //   shadow      occlusion of the NEE rays and their radiance (renderer.h:166-173)
 // so every kernel runs one material's code over a coherent batch. A sample's last
-// term, the emission of the miss or emitter that ends it, is kept apart (emit) and
-// added to the NEE terms (radiance) when the sample is banked: that is the
-// reference's order of additions (renderer.h:105-131 comes after the previous
-// bounce's NEE), and it lets bounce i's shadow rays run beside bounce i+1's
-// intersect. Queue pushes
+// term, the emission of the miss or emitter that ends it, is evaluated and added to
+// the NEE terms (radiance) when the sample is banked, from the path's last ray and
+// hit id (ended_emission): that is the reference's order of additions
+// (renderer.h:105-131 comes after the previous bounce's NEE), it lets bounce i's
+// shadow rays run beside bounce i+1's intersect, and it keeps the emission code out of
+// the traversal kernels. Queue pushes
 // cost one atomic per warp (ballot + popc). All path state is structure-of-arrays
 // indexed by pixel; queues hold pixel ids.
 #pragma once
@@ -50,8 +51,12 @@ __device__ __forceinline__ int warp_push(int *counter, bool want) {
 
 __device__ __forceinline__ s4 hero_wavelengths(const Job &job, float lambda0) {
     s4 l;
-    for (int k = 0; k < kHero; k++)
-        l.v[k] = job.lambda_min + fmodf(lambda0 - job.lambda_min + float(k) * job.lambda_range / kHero, job.lambda_range);
+    for (int k = 0; k < kHero; k++) {
+        // x mod range without the division loop: x is in [0, 2 range), where x - range is exact
+        float x = lambda0 - job.lambda_min + float(k) * job.lambda_range / kHero;
+        if (x >= job.lambda_range) x = x < 2 * job.lambda_range ? x - job.lambda_range : fmodf(x, job.lambda_range);
+        l.v[k] = job.lambda_min + x;
+    }
     return l;
 }
 
@@ -89,7 +94,7 @@ __device__ __forceinline__ void init_pixel(const PathState &ps, int p, const Job
     ps.path_info[p] = make_int2(local, job.depth);
     ps.film[p] = make_float4(0, 0, 0, 0);
     ps.radiance[p] = make_float4(0, 0, 0, 0);
-    ps.emit[p] = make_float4(0, 0, 0, 0);
+    ps.hit_id[p] = make_int4(0, kNoHit, 0, -1);
     ps.lam[p] = make_float4(job.lambda_min, job.lambda_min, job.lambda_min, job.lambda_min);
 }
 
@@ -135,14 +140,57 @@ LAMBDA_KERNEL void k_wave_prologue(int depth, PathState ps, cudaGraphConditional
     }
 }
 
+// Emission of the miss or emitter hit that ended path p's sample (renderer.h:105-131),
+// from its last ray and hit id; zero for a sample that ended otherwise (its last hit is
+// the material it was absorbed at) and before the first one.
+__device__ __forceinline__ s4 ended_emission(const DeviceScene &sc, const PathState &ps, int p, const s4 &lam) {
+    const int4 id = ps.hit_id[p];
+    if (id.y == kNoHit) return s4_fill(0);
+    const bool lights = sc.total_light_power > 0;
+    int4 m = make_int4(kEmissive, 0, 0, 0);
+    if (id.y != kMissed) m = __ldg(&sc.materials[id.x]);
+    if (m.x != kEmissive) return s4_fill(0);
+    const float4 o4 = ps.ray_o[p], d4 = ps.ray_d[p];
+    const f3 o = mk(o4.x, o4.y, o4.z), d = mk(d4.x, d4.y, d4.z);
+    const s4 T = from_f4(ps.throughput[p]);
+    const bool specular = d4.w != 0.0f;
+    const float prev_pdf = o4.w;
+    if (id.y == kMissed) {
+        float w = 1;
+        if (!specular && lights)
+            w = power_heuristic(prev_pdf, (1 / (4 * kPi)) * sc.light_power[sc.num_lights - 1] / sc.total_light_power);
+        return T * background_eval(sc, d, lam) * w;
+    }
+    const InstanceRef ir = instance_ref(sc, id.w);
+    Hit h;
+    closest_hit_finish(sc, make_ray(o, d), __int_as_float(id.z), id.y, id.w, h);
+    float w = 1;
+    if (!specular && lights) {
+        float M[16], Mi[16];
+        ir.load_m(M, 0);
+        ir.load_m(Mi, 1);
+        const Prim pr = load_prim(sc, id.y);
+        const f3 c0 = mk(M[0], M[4], M[8]);
+        const float light_power = prim_area(pr) * length_sq(c0) * sc.material_emission[id.x];
+        const float pdf = prim_pdf(pr, xform(Mi, o, 1), normalize(xform(Mi, d, 0)));
+        w = power_heuristic(prev_pdf, pdf * light_power / sc.total_light_power);
+    }
+    ShadePoint sp;
+    sp.point = h.point;
+    sp.u = h.u;
+    sp.v = h.v;
+    return T * spectrum_texture4(sc, m.y, sp, lam) * w;
+}
+
 // Radiance of a finished sample: its NEE terms, then the emission that ended it.
-__device__ __forceinline__ s4 sample_radiance(const PathState &ps, int p) {
-    return from_f4(ps.radiance[p]) + from_f4(ps.emit[p]);
+__device__ __forceinline__ s4 sample_radiance(const DeviceScene &sc, const PathState &ps, int p, const s4 &lam) {
+    return from_f4(ps.radiance[p]) + ended_emission(sc, ps, p, lam);
 }
 
 // Film += linear sRGB of pixel p's finished sample (renderer.h:84).
 __device__ __forceinline__ void bank_sample(const DeviceScene &sc, const PathState &ps, int p, const Job &job) {
-    const f3 rgb = spectrum_to_rgb(sc, sample_radiance(ps, p), from_f4(ps.lam[p]), job.lambda_range);
+    const s4 lam = from_f4(ps.lam[p]);
+    const f3 rgb = spectrum_to_rgb(sc, sample_radiance(sc, ps, p, lam), lam, job.lambda_range);
     float4 film = ps.film[p];
     film.x += rgb.x;
     film.y += rgb.y;
@@ -169,7 +217,6 @@ __device__ __forceinline__ void start_sample(const PathState &ps, int p, const J
     ps.ray_d[p] = make_float4(dir.x, dir.y, dir.z, 1.0f);
     ps.throughput[p] = make_float4(1, 1, 1, 1);
     ps.radiance[p] = make_float4(0, 0, 0, 0);
-    ps.emit[p] = make_float4(0, 0, 0, 0);
 }
 
 // Banks the finished sample of every pixel, then starts the next one.
@@ -185,7 +232,7 @@ LAMBDA_KERNEL void k_raygen(RenderParams rp, DeviceScene sc, PathState ps) {
     bank_sample(sc, ps, p, job);
     if (p >= n_now) {
         ps.radiance[p] = make_float4(0, 0, 0, 0);
-        ps.emit[p] = make_float4(0, 0, 0, 0);
+        ps.hit_id[p] = make_int4(0, kNoHit, 0, -1);
         return;
     }
     start_sample(ps, p, job, s);
@@ -198,19 +245,31 @@ __device__ __forceinline__ int material_of(const DeviceScene &sc, int inst_mater
     return inst_material >= 0 ? inst_material : prim_material(load_prim(sc, obj));
 }
 
-// Closest hit of path p (renderer.h:94-131). A miss or an emitter hit records the
-// path's emission term and returns -1: the path ends. Any other hit is stored for the
-// shade kernels and its material family returned: 0 Lambertian, 1 mirror or
-// dielectric, 2 thin film. The stored hit is (material, object, distance, instance)
-// alone: load_shade rebuilds the hit point, normal, (u, v) and facing from it with
-// the same functions, so the traversal kernels leave that work, and its bytes, to
-// the hits' shading kernels.
-__device__ __forceinline__ int trace_finish(const DeviceScene &sc, const PathState &ps, int p, const float4 &o4,
-                                            const float4 &d4, const Ray3 &wr, float best, int obj, int inst);
+// The emission used to be evaluated in the traversal kernels, which then spilled (64
+// registers, 336 B of spill loads); without it k_intersect runs the thin-film frame (B200,
+// 1080p, 16 spp) in 14.1 instead of 16.9 ms and the Cornell box's 144 launches in 2.6
+// instead of 3.1 ms, for 1.4 ms more in k_raygen on the former.
+// Stores path p's closest hit (best, obj, inst from the traversal, obj < 0 on a miss) and
+// returns its material family: 0 Lambertian, 1 mirror or dielectric, 2 thin film, or -1
+// when a miss or an emitter ends the path (ended_emission evaluates it when the sample
+// is banked). The stored hit is (material, object, distance, instance) alone:
+// load_shade and ended_emission rebuild the hit point, normal, (u, v) and facing from it,
+// so the traversal kernels leave that work, its bytes and its registers to others.
+__device__ __forceinline__ int store_hit(const DeviceScene &sc, const PathState &ps, int p, float best, int obj, int inst) {
+    if (obj < 0) {
+        ps.hit_id[p] = make_int4(0, kMissed, 0, -1);
+        return -1;
+    }
+    const int mat = material_of(sc, instance_ref(sc, inst).header().w, obj);
+    const int type = __ldg(&sc.materials[mat].x);
+    ps.hit_id[p] = make_int4(mat, obj, __float_as_int(best), inst);
+    return type == kLambertian ? 0 : (type == kThinFilm ? 2 : (type == kEmissive ? -1 : 1));
+}
 
+// Closest hit of path p (renderer.h:94-131), stored (store_hit).
 template <int K>
-__device__ __forceinline__ int trace_path(const DeviceScene &sc, const PathState &ps, int p, const WideStack &st_a,
-                                          const WideStack &st_b) {
+__device__ __forceinline__ int trace_path(const DeviceScene &sc, const PathState &ps, int p, const TravStack &st_a,
+                                          const TravStack &st_b) {
     const float4 o4 = ps.ray_o[p], d4 = ps.ray_d[p];
     const Ray3 wr = make_ray(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
     float best;
@@ -218,65 +277,15 @@ __device__ __forceinline__ int trace_path(const DeviceScene &sc, const PathState
     bool overflow = false;
     closest_hit_ids_w<K>(sc, wr, best, obj, inst, overflow, st_a, st_b);
     if (overflow) atomicOr(ps.error, 1);
-    return trace_finish(sc, ps, p, o4, d4, wr, best, obj, inst);
+    return store_hit(sc, ps, p, best, obj, inst);
 }
 
-// What trace_path does with path p's closest hit (ray o4, d4 = wr; best, obj, inst
-// from the traversal, obj < 0 on a miss): a miss or an emitter hit records the
-// emission term and returns -1; any other hit is stored and its material family
-// returned.
-__device__ __forceinline__ int trace_finish(const DeviceScene &sc, const PathState &ps, int p, const float4 &o4,
-                                            const float4 &d4, const Ray3 &wr, float best, int obj, int inst) {
-    const f3 o = mk(o4.x, o4.y, o4.z), d = mk(d4.x, d4.y, d4.z);
-    const bool specular = d4.w != 0.0f;
-    const float prev_pdf = o4.w;
-    const bool lights = sc.total_light_power > 0;
-    if (obj < 0) {
-        const s4 lam = from_f4(ps.lam[p]);
-        float w = 1;
-        if (!specular && lights)
-            w = power_heuristic(prev_pdf, (1 / (4 * kPi)) * sc.light_power[sc.num_lights - 1] / sc.total_light_power);
-        const s4 T = from_f4(ps.throughput[p]);
-        ps.emit[p] = to_f4(T * background_eval(sc, d, lam) * w);
-        return -1;
-    }
-    const InstanceRef ir = instance_ref(sc, inst);
-    const int4 ih = ir.header();
-    const int mat = material_of(sc, ih.w, obj);
-    const int4 m = __ldg(&sc.materials[mat]);
-    if (m.x == kEmissive) {
-        Hit h;
-        closest_hit_finish(sc, wr, best, obj, inst, h);
-        float w = 1;
-        if (!specular && lights) {
-            float M[16], Mi[16];
-            ir.load_m(M, 0);
-            ir.load_m(Mi, 1);
-            const Prim pr = load_prim(sc, obj);
-            const f3 c0 = mk(M[0], M[4], M[8]);
-            const float light_power = prim_area(pr) * length_sq(c0) * sc.material_emission[mat];
-            const float pdf = prim_pdf(pr, xform(Mi, o, 1), normalize(xform(Mi, d, 0)));
-            w = power_heuristic(prev_pdf, pdf * light_power / sc.total_light_power);
-        }
-        ShadePoint sp;
-        sp.point = h.point;
-        sp.u = h.u;
-        sp.v = h.v;
-        const s4 lam = from_f4(ps.lam[p]);
-        const s4 T = from_f4(ps.throughput[p]);
-        ps.emit[p] = to_f4(T * spectrum_texture4(sc, m.y, sp, lam) * w);
-        return -1;
-    }
-    ps.hit_id[p] = make_int4(mat, obj, __float_as_int(best), inst);
-    return m.x == kLambertian ? 0 : (m.x == kThinFilm ? 2 : 1);
-}
-
-// Closest hit; misses and emitter hits record their emission term and end the
-// path (renderer.h:105-131); other hits go to their material's queue.
+// Closest hit; a miss or an emitter hit ends the path (renderer.h:105-131); other hits
+// go to their material's queue.
 template <int K>
 LAMBDA_KERNEL void __launch_bounds__(256, 4) k_intersect(int bounce, RenderParams rp, DeviceScene sc, PathState ps) {
     extern __shared__ int stack_smem[];
-    WideStack st_a, st_b;
+    TravStack st_a, st_b;
     wide_stacks(stack_smem, sc, st_a, st_b);
     const int n = ps.counts[queue_slot(bounce, kQActive)];
     const int *q = ps.queue[bounce & 1];
@@ -295,102 +304,144 @@ LAMBDA_KERNEL void __launch_bounds__(256, 4) k_intersect(int bounce, RenderParam
     }
 }
 
-// Closest hits of the bounce's queue with rays taken lane by lane. Each lane keeps its
-// traversal (stacks, instance-space ray, best hit) across iterations of one loop and
-// advances it by one stack entry per iteration, in the order closest_hit_w visits
-// them, so its hits are closest_hit_w's bit for bit. A lane whose ray is done
-// finishes it as trace_path does, pushes it to its material queue with the lanes that
-// finish at the same step, and takes the next ray from the queue's fetch counter at
-// once. Lanes on different rays then step together instead of waiting for a warp's
-// longest ray. The loop ends when the queue is drained: every iteration pops an
-// entry, finishes a ray or takes one.
-template <int K>
+// A traversal lane takes the next work index of its queue: the lanes that need one
+// take consecutive indices, one atomic per group.
+__device__ __forceinline__ int take_next(int *next) {
+    const int lane = threadIdx.x & 31;
+    const unsigned need = __activemask();
+    const int leader = __ffs(need) - 1;
+    int base = 0;
+    if (lane == leader) base = atomicAdd(next, __popc(need));
+    base = __shfl_sync(need, base, leader);
+    return base + __popc(need & ((1u << lane) - 1u));
+}
+
+// The end of path p's closest hit in the lane-by-lane kernel: store_hit, then its
+// push to its material queue with the lanes that finish at the same step.
+__device__ __forceinline__ void fetch_finish(const DeviceScene &sc, const PathState &ps, int bounce, int p, float best,
+                                             int obj, int inst, bool overflow) {
+    if (overflow) atomicOr(ps.error, 1);
+    const int family = store_hit(sc, ps, p, best, obj, inst);
+    if (family >= 0) {
+        const int lane = threadIdx.x & 31;
+        const unsigned grp = __match_any_sync(__activemask(), family);
+        const int leader = __ffs(grp) - 1;
+        int base = 0;
+        if (lane == leader) base = atomicAdd(&ps.counts[queue_slot(bounce, kQLambert + family)], __popc(grp));
+        base = __shfl_sync(grp, base, leader);
+        ps.mat_queue[family][base + __popc(grp & ((1u << lane) - 1u))] = p;
+    }
+}
+
+// Closest hits of the bounce's queue with rays taken lane by lane: each lane keeps its
+// walk across iterations of one loop and advances it by one node per iteration; a
+// lane whose ray is done finishes it as trace_path does and takes the next ray from
+// the queue's fetch counter at once, so lanes on different rays step together
+// instead of waiting for a warp's longest ray. Over the exact layouts TLAS and BLAS
+// nodes step through the same code (FlatWalk), so that lanes at different levels do not
+// run in turn: 10,000 instances of a 100,000-triangle mesh (B200, 960x540, 1 spp,
+// intersect) 25.1 -> 24.2 ms. Visiting the nearest child first instead took 11.8 ms there,
+// but its hits equal the fixed order's only while no primitive's computed distance
+// lies before its own box, which rays within about 1e-3 of a triangle's plane can
+// break, so the fixed order stays.
+template <int L>
 LAMBDA_KERNEL void __launch_bounds__(256, 2) k_intersect_fetch(int bounce, RenderParams rp, DeviceScene sc,
                                                                PathState ps) {
     extern __shared__ int stack_smem[];
-    WideStack st, sub;
+    TravStack st, sub;
     wide_stacks(stack_smem, sc, st, sub);
     const int n = ps.counts[queue_slot(bounce, kQActive)];
     const int *q = ps.queue[bounce & 1];
     int *next = &ps.counts[queue_slot(bounce, kQFetch)];
-    const int lane = threadIdx.x & 31;
     int p = -1;
-    Ray3 wr, lr;
-    float best = kMax;
-    int best_obj = -1, best_inst = -1, inst = -1, sp = 0, ssp = 0;
+    Ray3 wr;
     bool overflow = false;
-    for (;;) {
-        if (p < 0) {
-            // the lanes that need a ray take consecutive entries, one atomic per group
-            const unsigned need = __activemask();
-            const int leader = __ffs(need) - 1;
-            int base = 0;
-            if (lane == leader) base = atomicAdd(next, __popc(need));
-            base = __shfl_sync(need, base, leader);
-            const int idx = base + __popc(need & ((1u << lane) - 1u));
-            if (idx >= n) break;
-            p = q[idx];
-            const float4 o4 = ps.ray_o[p], d4 = ps.ray_d[p];
-            wr = make_ray(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
-            best = kMax;
-            best_obj = best_inst = -1;
-            sp = ssp = 0;
-            overflow = false;
-            float te;
-            if (slab(__ldg(&sc.nodes[0]), __ldg(&sc.nodes[1]), wr, te))
-                st.put(sp++, root_entry<K>(sc, __ldg(&sc.wide_code[0])), te);
-        } else if (ssp > 0 && !overflow) {
-            // one BLAS entry
-            --ssp;
-            float te2 = sub.te[ssp * sub.stride];
-            const int c2 = pop_code<K>(sc, sub.code[ssp * sub.stride], te2, lr, best);
-            if (c2 != INT_MIN) {
-                if (c2 >= 0) {
-                    ssp = wide_expand<K>(sc, c2, lr, best, sub, ssp, overflow);
-                } else {
-                    const int2 lf = __ldg(&sc.wide_leaves[-c2 - 1]);
-                    for (int k = 0; k < lf.y; k++) {
-                        const float t = intersect_t(load_prim(sc, lf.x + k), lr, best);
-                        if (t >= 0) {
-                            best = t;
-                            best_obj = lf.x + k;
-                            best_inst = inst;
+    if constexpr (!kQuantOf<L>) {
+        const TravStack both = trav_stack(st, sub);
+        FlatWalk w;
+        bool walking = false;
+        for (;;) {
+            if (p < 0) {
+                const int idx = take_next(next);
+                if (idx >= n) break;
+                p = q[idx];
+                const float4 o4 = ps.ray_o[p], d4 = ps.ray_d[p];
+                wr = make_ray(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+                overflow = false;
+                walking = flat_start(sc, wr, w);
+            } else if (walking) {
+                walking = flat_step<L>(sc, wr, w, both, overflow);
+            } else {
+                fetch_finish(sc, ps, bounce, p, w.best, w.obj, w.hit_inst, overflow);
+                p = -1;
+            }
+        }
+    } else {
+        Ray3 lr;
+        float best = kMax;
+        int best_obj = -1, best_inst = -1, inst = -1, sp = 0, ssp = 0;
+        for (;;) {
+            if (p < 0) {
+                const int idx = take_next(next);
+                if (idx >= n) break;
+                p = q[idx];
+                const float4 o4 = ps.ray_o[p], d4 = ps.ray_d[p];
+                wr = make_ray(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+                best = kMax;
+                best_obj = best_inst = -1;
+                sp = ssp = 0;
+                overflow = false;
+                float te;
+                if (slab(__ldg(&sc.nodes[0]), __ldg(&sc.nodes[1]), wr, te))
+                    st.put(sp++, root_entry<L>(sc, __ldg(&sc.wide_code[0])), te);
+            } else if (ssp > 0 && !overflow) {
+                // one BLAS entry
+                --ssp;
+                float te2;
+                int c2;
+                sub.get(ssp, c2, te2);
+                c2 = pop_code<L>(sc, c2, te2, lr, best);
+                if (c2 != INT_MIN) {
+                    if (c2 >= 0) {
+                        ssp = wide_expand<L>(sc, c2, lr, best, sub, ssp, overflow);
+                    } else {
+                        const int2 lf = __ldg(&sc.wide_leaves[-c2 - 1]);
+                        for (int k = 0; k < lf.y; k++) {
+                            const float t = intersect_t(load_prim(sc, lf.x + k), lr, best);
+                            if (t >= 0) {
+                                best = t;
+                                best_obj = lf.x + k;
+                                best_inst = inst;
+                            }
                         }
                     }
                 }
-            }
-        } else if (sp > 0 && !overflow) {
-            // one TLAS entry; a leaf starts its instance's BLAS (the first instance only)
-            --sp;
-            float te = st.te[sp * st.stride];
-            const int code = pop_code<K>(sc, st.code[sp * st.stride], te, wr, best);
-            if (code != INT_MIN) {
-                if (code >= 0) {
-                    sp = wide_expand<K>(sc, code, wr, best, st, sp, overflow);
-                } else {
-                    inst = __ldg(&sc.wide_leaves[-code - 1]).x;
-                    const uint32_t flags = sc.instance_flags[inst];
-                    const InstanceRef ir = instance_ref(sc, inst);
-                    const int root = ir.header().z;
-                    lr = to_local(flags, ir, wr);
-                    if ((flags & 2u) ||
-                        (slab(__ldg(&sc.nodes[2 * root]), __ldg(&sc.nodes[2 * root + 1]), lr, te) && !(te > best)))
-                        sub.put(ssp++, root_entry<K>(sc, __ldg(&sc.wide_code[root])), te);
+            } else if (sp > 0 && !overflow) {
+                // one TLAS entry; a leaf starts its instance's BLAS (the first instance only)
+                --sp;
+                float te;
+                int code;
+                st.get(sp, code, te);
+                code = pop_code<L>(sc, code, te, wr, best);
+                if (code != INT_MIN) {
+                    if (code >= 0) {
+                        sp = wide_expand<L>(sc, code, wr, best, st, sp, overflow);
+                    } else {
+                        inst = __ldg(&sc.wide_leaves[-code - 1]).x;
+                        const uint32_t flags = sc.instance_flags[inst];
+                        const InstanceRef ir = instance_ref(sc, inst);
+                        const int root = ir.header().z;
+                        lr = to_local(flags, ir, wr);
+                        if ((flags & 2u) ||
+                            (slab(__ldg(&sc.nodes[2 * root]), __ldg(&sc.nodes[2 * root + 1]), lr, te) && !(te > best)))
+                            sub.put(ssp++, root_entry<L>(sc, __ldg(&sc.wide_code[root])), te);
+                    }
                 }
+            } else {
+                // the ray is done (or a stack overflowed): finish it and push it
+                fetch_finish(sc, ps, bounce, p, best, best_obj, best_inst, overflow);
+                p = -1;
             }
-        } else {
-            // the ray is done (or a stack overflowed): finish it and push it
-            if (overflow) atomicOr(ps.error, 1);
-            const int family = trace_finish(sc, ps, p, ps.ray_o[p], ps.ray_d[p], wr, best, best_obj, best_inst);
-            if (family >= 0) {
-                const unsigned grp = __match_any_sync(__activemask(), family);
-                const int leader = __ffs(grp) - 1;
-                int base = 0;
-                if (lane == leader) base = atomicAdd(&ps.counts[queue_slot(bounce, kQLambert + family)], __popc(grp));
-                base = __shfl_sync(grp, base, leader);
-                ps.mat_queue[family][base + __popc(grp & ((1u << lane) - 1u))] = p;
-            }
-            p = -1;
         }
     }
 }
@@ -415,7 +466,7 @@ __device__ __forceinline__ ShadeIn load_shade(const PathState &ps, const DeviceS
     s.p = p;
     const float4 o4 = ps.ray_o[p], d4 = ps.ray_d[p];
     s.d = mk(d4.x, d4.y, d4.z);
-    // the hit record from (object, distance, instance), as closest_hit_w makes it
+    // the hit record from (object, distance, instance), as the traversal leaves it
     const int4 id = ps.hit_id[p];
     Hit h;
     closest_hit_finish(sc, make_ray(mk(o4.x, o4.y, o4.z), s.d), __int_as_float(id.z), id.y, id.w, h);
@@ -784,8 +835,8 @@ __device__ __forceinline__ void shadow_finish(const DeviceScene &sc, const PathS
 
 // The NEE shadow ray of path p: occlusion, then shadow_finish.
 template <int K>
-__device__ __forceinline__ void shadow_path(const DeviceScene &sc, const PathState &ps, int p, const WideStack &st_a,
-                                            const WideStack &st_b) {
+__device__ __forceinline__ void shadow_path(const DeviceScene &sc, const PathState &ps, int p, const TravStack &st_a,
+                                            const TravStack &st_b) {
     const float4 o = ps.sh_o[p], dd = ps.sh_d[p];
     const int2 light = ps.sh_light[p];
     Hit lh;
@@ -797,7 +848,7 @@ __device__ __forceinline__ void shadow_path(const DeviceScene &sc, const PathSta
 template <int K>
 LAMBDA_KERNEL void __launch_bounds__(256, 4) k_shadow(int bounce, RenderParams rp, DeviceScene sc, PathState ps) {
     extern __shared__ int stack_smem[];
-    WideStack st_a, st_b;
+    TravStack st_a, st_b;
     wide_stacks(stack_smem, sc, st_a, st_b);
     const int n = ps.counts[queue_slot(bounce, kQShadow)];
     const int stride = gridDim.x * blockDim.x;
@@ -816,7 +867,7 @@ LAMBDA_KERNEL void __launch_bounds__(256, 4) k_shadow(int bounce, RenderParams r
 template <int K>
 LAMBDA_KERNEL void __launch_bounds__(256, 2) k_shadow_fetch(int bounce, RenderParams rp, DeviceScene sc, PathState ps) {
     extern __shared__ int stack_smem[];
-    WideStack st, sub;
+    TravStack st, sub;
     wide_stacks(stack_smem, sc, st, sub);
     const int n = ps.counts[queue_slot(bounce, kQShadow)];
     int *next = &ps.counts[queue_slot(bounce, kQShadowFetch)];
@@ -866,8 +917,10 @@ LAMBDA_KERNEL void __launch_bounds__(256, 2) k_shadow_fetch(int bounce, RenderPa
         } else if (!occ && ssp > 0) {
             // one BLAS entry; any primitive other than the light closer than it occludes
             --ssp;
-            float te2 = sub.te[ssp * sub.stride];
-            const int c2 = pop_code<K>(sc, sub.code[ssp * sub.stride], te2, lr, best);
+            float te2;
+            int c2;
+            sub.get(ssp, c2, te2);
+            c2 = pop_code<K>(sc, c2, te2, lr, best);
             if (c2 != INT_MIN) {
                 if (c2 >= 0) {
                     ssp = wide_expand<K>(sc, c2, lr, best, sub, ssp, overflow);
@@ -883,8 +936,10 @@ LAMBDA_KERNEL void __launch_bounds__(256, 2) k_shadow_fetch(int bounce, RenderPa
         } else if (!occ && sp > 0) {
             // one TLAS entry; a leaf starts its instance's BLAS (the first instance only)
             --sp;
-            float te = st.te[sp * st.stride];
-            const int code = pop_code<K>(sc, st.code[sp * st.stride], te, wr, best);
+            float te;
+            int code;
+            st.get(sp, code, te);
+            code = pop_code<K>(sc, code, te, wr, best);
             if (code != INT_MIN) {
                 if (code >= 0) {
                     sp = wide_expand<K>(sc, code, wr, best, st, sp, overflow);
@@ -919,7 +974,7 @@ LAMBDA_KERNEL void __launch_bounds__(256, 2) k_shadow_fetch(int bounce, RenderPa
 template <int K, bool kFp64>
 LAMBDA_KERNEL void __launch_bounds__(256, 3) k_bounce(int bounce, RenderParams rp, DeviceScene sc, PathState ps) {
     extern __shared__ int stack_smem[];
-    WideStack st_a, st_b;
+    TravStack st_a, st_b;
     wide_stacks(stack_smem, sc, st_a, st_b);
     const int n = ps.counts[queue_slot(bounce, kQActive)];
     const int *q = ps.queue[bounce & 1];
@@ -951,7 +1006,8 @@ LAMBDA_KERNEL void __launch_bounds__(256, 3) k_bounce(int bounce, RenderParams r
 // Last sample of pixel p into the film, then the average (renderer.h:84-91), into
 // the job's own image.
 __device__ __forceinline__ void finish_pixel(const DeviceScene &sc, const PathState &ps, int p, const Job &job) {
-    const f3 rgb = spectrum_to_rgb(sc, sample_radiance(ps, p), from_f4(ps.lam[p]), job.lambda_range);
+    const s4 lam = from_f4(ps.lam[p]);
+    const f3 rgb = spectrum_to_rgb(sc, sample_radiance(sc, ps, p, lam), lam, job.lambda_range);
     float4 film = ps.film[p];
     film.x += rgb.x;
     film.y += rgb.y;
@@ -983,7 +1039,7 @@ template <int K, bool kFp64>
 LAMBDA_KERNEL void __launch_bounds__(256, 3) k_path(RenderParams rp, DeviceScene sc, PathState ps, int *work, int *done,
                                                  int *progress) {
     extern __shared__ int stack_smem[];
-    WideStack st_a, st_b;
+    TravStack st_a, st_b;
     wide_stacks(stack_smem, sc, st_a, st_b);
     const int lane = threadIdx.x & 31;
     unsigned n_seg = 0, n_nee = 0, n_film = 0, n_lam = 0, n_spec = 0;
