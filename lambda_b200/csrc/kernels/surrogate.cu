@@ -468,9 +468,7 @@ __global__ void k_film_labels(uint64_t seed, int64_t first, int n, Range rg, flo
     float v[kIn];
     for (int d = 0; d < kIn; d++)
         v[d] = float(rg.lo[d] + (rg.hi[d] - rg.lo[d]) * uniform01(seed, uint64_t(first + i), d));
-    cx<double> idx[3] = {cx<double>{1.0, 0.0}, cx<double>{double(v[3]), 0.0}, cx<double>{double(v[4]), 0.0}};
-    const double d = v[2];
-    const FilmResult<double> r = film_stack<double, 1>(1, idx, &d, double(v[1]), double(v[0]));
+    const FilmResult<double> r = film_single_fp64(1.0, double(v[3]), double(v[4]), double(v[2]), double(v[1]), double(v[0]));
     float e[kIn];
     encode(v, rg, e);
     for (int k = 0; k < kIn; k++) x[size_t(i) * kRowStride + k] = e[k];

@@ -307,4 +307,98 @@ __device__ __forceinline__ R film_reflectance_stream(int L, IndexOf index_of, co
     return (rs2 + rp2) * R(0.5);
 }
 
+// One film with real indices in FP64. Each cosine is then real or, past a critical angle,
+// +i times a real number (csqrt_'s branch for the +0 imaginary parts that the general
+// product meets), and the first row of the product of the three 2x2 matrices has the
+// closed form
+//   M01 / M00 = (r12 + r01 e) / (1 + r01 r12 e),  e = e^{2 i phi}
+// per polarisation with complex Fresnel amplitudes r01 and r12 of the two interfaces;
+// e lies on the unit circle, or is real where the film itself is evanescent. The squared
+// modulus is taken from both parts (no cancellation where the reflectance vanishes). Per
+// wavelength that is one sincos (or exp) and a division per polarisation, in place of six
+// complex matrix entries with their complex divisions, square roots and exponentials.
+// Measured (B200): labels of 2 x 262,144 training and audit samples 102 -> 41 us, the FP64
+// film shade of a 641 x 363 frame at 9 spp 9.4 -> 3.0 ms (7.4 ms with the closed form only
+// where no angle is past critical: one lane past it holds its warp).
+struct FilmReal {
+    double n1, c1;                    // the film's index and cosine (its imaginary part if evanescent)
+    bool evanescent;
+    cx<double> rs01, rs12, rp01, rp12;
+    double ts, tp;                    // |t01 t12|^2 Re(n2 c2) / (n0 c0)
+};
+
+// Fresnel amplitude (a - b) / (a + b); tt gets |2 a / (a + b)|^2.
+__device__ __forceinline__ cx<double> film_real_fresnel(cx<double> a, cx<double> b, double &tt) {
+    const double sr = a.re + b.re, si = a.im + b.im, inv = 1.0 / (sr * sr + si * si);
+    tt = 4.0 * (a.re * a.re + a.im * a.im) * inv;
+    return cx<double>{((a.re - b.re) * sr + (a.im - b.im) * si) * inv, 2.0 * (a.im * b.re - a.re * b.im) * inv};
+}
+
+// False where the closed form is not taken (the general product is then formed): a
+// cosine of incidence outside (0, 1], an index that is not positive, or a film cosine of 0.
+__device__ __forceinline__ bool film_real_prepare(double n0, double n1, double n2, double c0, FilmReal &f) {
+    if (!(c0 > 0.0 && c0 <= 1.0 && n0 > 0.0 && n1 > 0.0 && n2 > 0.0)) return false;
+    const double q01 = n0 / n1, q12 = n1 / n2;
+    const double sin1 = q01 * (q01 * (1.0 - c0 * c0));  // sin^2 in the film
+    const double sin2 = q12 * (q12 * sin1);             // and in the substrate
+    const double c1 = sqrt(fabs(1.0 - sin1)), c2 = sqrt(fabs(1.0 - sin2));
+    if (!(c1 > 0.0)) return false;
+    f.n1 = n1;
+    f.c1 = c1;
+    f.evanescent = sin1 > 1.0;
+    const cx<double> k0{c0, 0.0}, k1{f.evanescent ? 0.0 : c1, f.evanescent ? c1 : 0.0};
+    const cx<double> k2{sin2 > 1.0 ? 0.0 : c2, sin2 > 1.0 ? c2 : 0.0};
+    double s01, s12, p01, p12;
+    f.rs01 = film_real_fresnel(k0 * n0, k1 * n1, s01);
+    f.rs12 = film_real_fresnel(k1 * n1, k2 * n2, s12);
+    f.rp01 = film_real_fresnel(k0 * n1, k1 * n0, p01);
+    f.rp12 = film_real_fresnel(k1 * n2, k2 * n1, p12);
+    // t = 2 n_a c_a / (...): the p amplitudes above carry the other medium's index
+    const double g = n2 * k2.re / (n0 * c0);
+    f.ts = g * s01 * s12;
+    f.tp = g * p01 * p12 * (n0 / n1) * (n0 / n1) * (n1 / n2) * (n1 / n2);
+    return true;
+}
+
+// |(r12 + r01 e) / (1 + r01 r12 e)|^2; den: |1 + r01 r12 e|^2.
+__device__ __forceinline__ double film_real_r(cx<double> r01, cx<double> r12, cx<double> e, double &den) {
+    const cx<double> u = r01 * e, n = r12 + u, w = r12 * u;
+    const double dr = 1.0 + w.re;
+    den = dr * dr + w.im * w.im;
+    return cabs2(n) / den;
+}
+
+// Reflectances at one wavelength (k = 2 pi / lambda, thickness d) and, with want_t, the
+// transmittances. False past the decay at which the general product overflows its
+// exponentials' useful range.
+__device__ __forceinline__ bool film_real_apply(const FilmReal &f, double d, double k, bool want_t, FilmResult<double> &out) {
+    const double phase = 2.0 * (((f.n1 * k) * d) * f.c1);
+    cx<double> e;
+    double decay = 1.0;
+    if (f.evanescent) {
+        if (!(fabs(phase) < 600.0)) return false;
+        e = cx<double>{exp(-phase), 0.0};
+        decay = e.re;
+    } else {
+        sincos(phase, &e.im, &e.re);
+    }
+    double ds, dp;
+    out.rs = film_real_r(f.rs01, f.rs12, e, ds);
+    out.rp = film_real_r(f.rp01, f.rp12, e, dp);
+    out.ts = want_t ? f.ts * decay / ds : 0.0;
+    out.tp = want_t ? f.tp * decay / dp : 0.0;
+    return true;
+}
+
+// A single-film query with real indices in FP64: the closed form, else the general product.
+__device__ __forceinline__ FilmResult<double> film_single_fp64(double n0, double n1, double n2, double d, double cos0,
+                                                               double lambda) {
+    FilmReal f;
+    FilmResult<double> r;
+    if (film_real_prepare(n0, n1, n2, cos0, f) && film_real_apply(f, d, 2.0 * 3.14159265358979323846 / lambda, true, r))
+        return r;
+    const cx<double> idx[3] = {cx<double>{n0, 0.0}, cx<double>{n1, 0.0}, cx<double>{n2, 0.0}};
+    return film_stack<double, 1>(1, idx, &d, cos0, lambda);
+}
+
 }  // namespace lambda_dev

@@ -701,11 +701,32 @@ __device__ inline s4 thin_film_r4(const DeviceScene &sc, const int4 &m, bool fro
 }
 
 // Thin-film reflectance as the reference evaluates it (material.h:263-309): complex
-// double characteristic matrices from the complex spectra, k = 2 pi / lambda formed
-// in float, |r| rounded to float and squared in float.
+// double characteristic matrices from the complex spectra (their closed form for one
+// film with real, non-dispersive indices), k = 2 pi / lambda formed in float, |r|
+// rounded to float and squared in float.
 __device__ inline s4 thin_film_r4_fp64(const DeviceScene &sc, const int4 &m, bool front, float cos0, const s4 &lam,
-                                       const float *thickness) {
+                                       const float *thickness, float4 ff = make_float4(0, 0, 0, 0)) {
     const int L = m.y < kMaxFilmLayers ? m.y : kMaxFilmLayers;
+    if (ff.w != 0.0f) {
+        // one film with real, non-dispersive indices (film_flat)
+        auto index_of = [&](int k) { return cspectrum_at(sc, sc.material_props[m.z + k], lam.v[0]).x; };
+        const double na = index_of(0), nb = index_of(1), nc = index_of(2);
+        FilmReal f;
+        if (film_real_prepare(front ? na : nc, nb, front ? nc : na, double(cos0), f)) {
+            s4 R;
+            bool ok = true;
+#pragma unroll 1
+            for (int w = 0; w < kHero; w++) {
+                FilmResult<double> r;
+                ok = ok && film_real_apply(f, double(thickness[0]), double((2 * kPi) / lam.v[w]), false, r);
+                float rs = float(sqrt(r.rs)), rp = float(sqrt(r.rp));
+                rs *= rs;
+                rp *= rp;
+                R.v[w] = (rs + rp) * 0.5f;
+            }
+            if (ok) return R;
+        }
+    }
     double d[kMaxFilmLayers];
     for (int k = 0; k < L; k++) d[k] = double(thickness[front ? k : L - 1 - k]);
     s4 R;
@@ -773,7 +794,7 @@ __device__ __forceinline__ bool film_path(const DeviceScene &sc, const PathState
     float thick[kMaxFilmLayers];
     thin_film_thickness(sc, s, thick);
     const float4 ff = __ldg(&sc.film_flat[s.mat]);
-    const s4 R = kFp64 ? thin_film_r4_fp64(sc, s.m, s.front, dot(s.nrm, -s.d), s.lam, thick)
+    const s4 R = kFp64 ? thin_film_r4_fp64(sc, s.m, s.front, dot(s.nrm, -s.d), s.lam, thick, ff)
                        : thin_film_r4(sc, s.m, s.front, dot(s.nrm, -s.d), s.lam, thick, ff);
     Rng rng = path_rng(ps, p);
     s4 att;
