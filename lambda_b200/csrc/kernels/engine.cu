@@ -71,6 +71,24 @@ cudaError_t DeviceBuffer::upload(const void *src, size_t n, cudaStream_t st) {
     return cudaMemcpyAsync(ptr, src, n, cudaMemcpyHostToDevice, st);
 }
 
+void HostBuffer::release() {
+    if (ptr) cudaFreeHost(ptr);
+    ptr = nullptr;
+    bytes = 0;
+}
+
+cudaError_t HostBuffer::reserve(size_t n) {
+    if (n <= bytes) return cudaSuccess;
+    release();
+    cudaError_t e = cudaHostAlloc(&ptr, n, cudaHostAllocDefault);
+    if (e != cudaSuccess) {
+        ptr = nullptr;
+        return e;
+    }
+    bytes = n;
+    return cudaSuccess;
+}
+
 bool is_device_pointer(const void *p) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
@@ -146,6 +164,7 @@ lambda_ctx::~lambda_ctx() {
     if (stream) cudaStreamSynchronize(stream);
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     if (progress_host) cudaFreeHost(progress_host);
+    io.release();
     for (DeviceBuffer *b : all_buffers()) b->release();
     if (ev_start) cudaEventDestroy(ev_start);
     if (ev_stop) cudaEventDestroy(ev_stop);
@@ -663,6 +682,9 @@ cudaError_t StageProfiler::collect() {
     return cudaSuccess;
 }
 
+// A pass's statistics and, after them, its error flags: one clear and one copy back.
+constexpr size_t kPassStats = 8, kPassStatBytes = kPassStats * 8 + 16;
+
 lambda_status lambda_ctx::ensure_state(int pixels, int depth) {
     lambda_ctx *ctx = this;
     const size_t P = size_t(pixels);
@@ -688,8 +710,7 @@ lambda_status lambda_ctx::ensure_state(int pixels, int depth) {
     CK(r.qm2.reserve(P * 4), "allocate queues");
     CK(r.counts.reserve(size_t(kQueues * (depth + 2)) * 4), "allocate queues");
     CK(r.wave.reserve(16), "allocate queues");
-    CK(r.stats.reserve(8 * 8), "allocate statistics");
-    CK(r.error.reserve(16), "allocate flags");
+    CK(r.stats.reserve(kPassStatBytes), "allocate statistics");
     PathState &ps = pstate;
     ps.rng = r.rng.as<uint64_t>();
     ps.film = r.film.as<float4>();
@@ -713,7 +734,7 @@ lambda_status lambda_ctx::ensure_state(int pixels, int depth) {
     ps.counts = r.counts.as<int>();
     ps.wave = r.wave.as<int>();
     ps.stats = r.stats.as<unsigned long long>();
-    ps.error = r.error.as<int>();
+    ps.error = reinterpret_cast<int *>(ps.stats + kPassStats);  // read back together
     return LAMBDA_OK;
 }
 
@@ -777,7 +798,22 @@ struct RenderTotals {
     int err = 0;
 };
 
-// Renders jobs[order[first..last)] as one wavefront pass (see lambda_render_batch).
+// What identifies a pass's launch plan, compared byte by byte.
+struct PlanKey {
+    RenderParams rp;
+    DeviceScene sc;
+    PathState ps;
+    lambda_tuning tuning;
+    lambda_limits limits;
+    lambda_film_range range;
+    const void *surrogate[4];
+    int waves, mode;
+};
+
+// Renders jobs[order[first..last)] as one wavefront pass (see lambda_render_batch). A pass
+// shaped like the context's last one launches that one's graph again: capturing,
+// instantiating and configuring about 100 kernel nodes took 0.2 to 0.4 ms per call on
+// the host, as long as a small frame takes on the GPU.
 lambda_status render_pass(lambda_ctx *ctx, const lambda_job *jobs, const std::vector<int> &order, size_t first,
                           size_t last, bool surrogate, bool fp64, StageProfiler *prof, volatile int32_t *completed,
                           int32_t completed_base, int32_t completed_total, RenderTotals &tot) {
@@ -834,26 +870,50 @@ lambda_status render_pass(lambda_ctx *ctx, const lambda_job *jobs, const std::ve
         work[i] = make_int2(by_cost[i], int(wbase));
         wbase += int64_t(dj[by_cost[i]].width) * dj[by_cost[i]].height;
     }
-    CK(r.jobs.reserve(nj * sizeof(Job)), "allocate job table");
-    CK(r.active.reserve(active.size() * 4), "allocate job table");
-    CK(r.work.reserve(nj * sizeof(int2)), "allocate job table");
+    // the job table, the active prefixes and the work order go up in one copy from
+    // page-locked memory, which also receives the statistics
+    const size_t at_active = (nj * sizeof(Job) + 15) / 16 * 16, at_work = at_active + (active.size() * 4 + 15) / 16 * 16;
+    const size_t table = at_work + nj * sizeof(int2);
+    CK(r.jobs.reserve(table), "allocate job table");
+    CK(ctx->io.reserve(128 + table), "allocate job table");
+    char *const host_stats = static_cast<char *>(ctx->io.ptr), *const host_table = host_stats + 128;
+    std::memcpy(host_table, dj.data(), nj * sizeof(Job));
+    std::memcpy(host_table + at_active, active.data(), active.size() * 4);
+    std::memcpy(host_table + at_work, work.data(), nj * sizeof(int2));
     cudaStream_t stream = ctx->stream;
-    CK(cudaMemcpyAsync(r.jobs.ptr, dj.data(), nj * sizeof(Job), cudaMemcpyHostToDevice, stream), "upload job table");
-    CK(cudaMemcpyAsync(r.active.ptr, active.data(), active.size() * 4, cudaMemcpyHostToDevice, stream),
-       "upload job table");
-    CK(cudaMemcpyAsync(r.work.ptr, work.data(), nj * sizeof(int2), cudaMemcpyHostToDevice, stream), "upload job table");
+    CK(cudaMemcpyAsync(r.jobs.ptr, host_table, table, cudaMemcpyHostToDevice, stream), "upload job table");
 
     RenderParams rp{};
     rp.jobs = r.jobs.as<Job>();
     rp.num_jobs = int(nj);
     rp.num_pixels = P;
     rp.depth_max = d_max;
-    rp.active = r.active.as<int>();
-    rp.work = r.work.as<int2>();
+    rp.active = reinterpret_cast<int *>(r.jobs.as<char>() + at_active);
+    rp.work = reinterpret_cast<int2 *>(r.jobs.as<char>() + at_work);
 
     const PathState ps = ctx->pstate;
     const lambda_tuning &tu = ctx->tuning;
     const DeviceScene sc = ctx->scene_view(tu.bvh_width);
+    // Everything a pass's graph is made of: the arguments of its kernels, all in the
+    // context's own buffers, and what chooses the kernels, their grids and the wave count.
+    PlanKey key;
+    std::memset(static_cast<void *>(&key), 0, sizeof(key));
+    key.rp = rp;
+    key.sc = sc;
+    key.ps = ps;
+    key.tuning = tu;
+    key.limits = ctx->limits;
+    key.waves = s_max;
+    key.mode = (surrogate ? 1 : 0) | (fp64 ? 2 : 0);
+    if (surrogate) {
+        key.range = ctx->surrogate_range;
+        key.surrogate[0] = ctx->sbuf.weights_bf16.ptr;
+        key.surrogate[1] = r.film_rows.ptr;
+        key.surrogate[2] = r.film_out.ptr;
+        key.surrogate[3] = r.film_in_domain.ptr;
+    }
+    const bool reuse = !prof && ctx->graph_exec && ctx->plan_key.size() == sizeof(key) &&
+                       std::memcmp(ctx->plan_key.data(), &key, sizeof(key)) == 0;
     const int dev = ctx->device, sms = ctx->sm_count;
     const int tb = tu.trace_block, sb = tu.shade_block, gs = tu.grid_scale;
     const size_t stack_smem = wide_stack_bytes(tb, sc.stack_tlas, sc.stack_blas);
@@ -872,16 +932,21 @@ lambda_status render_pass(lambda_ctx *ctx, const lambda_job *jobs, const std::ve
     static const IntersectKernel bounce64[6] = {k_bounce<2, true>, k_bounce<4, true>, k_bounce<8, true>, k_bounce<2 | kCompressed, true>, k_bounce<4 | kCompressed, true>, k_bounce<8 | kCompressed, true>}, bounce32[6] = {k_bounce<2, false>, k_bounce<4, false>, k_bounce<8, false>, k_bounce<2 | kCompressed, false>, k_bounce<4 | kCompressed, false>, k_bounce<8 | kCompressed, false>};
     const bool fused = tu.fused_bounce != 0 && !surrogate;
     const IntersectKernel k_bnc = fp64 ? bounce64[li] : bounce32[li];
+    // Every kernel may use all the shared memory a block can have: a limit set to one
+    // scene's stacks could fall below what a kept plan of another context launches with.
     int smem_optin = 0;
-    CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "device attribute");
-    if (stack_smem > size_t(smem_optin))
-        return ctx->fail(LAMBDA_ERR_UNSUPPORTED, "the scene's traversal stacks exceed shared memory at this block size");
-    CK(cudaFuncSetAttribute(f_isect, cudaFuncAttributeMaxDynamicSharedMemorySize, int(stack_smem)), "configure kernels");
-    CK(cudaFuncSetAttribute(f_shadow, cudaFuncAttributeMaxDynamicSharedMemorySize, int(stack_smem)), "configure kernels");
-    if (fused)
-        CK(cudaFuncSetAttribute((const void *)k_bnc, cudaFuncAttributeMaxDynamicSharedMemorySize, int(stack_smem)),
-           "configure kernels");
+    if (!reuse) {
+        CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "device attribute");
+        if (stack_smem > size_t(smem_optin))
+            return ctx->fail(LAMBDA_ERR_UNSUPPORTED, "the scene's traversal stacks exceed shared memory at this block size");
+        CK(cudaFuncSetAttribute(f_isect, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin), "configure kernels");
+        CK(cudaFuncSetAttribute(f_shadow, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin), "configure kernels");
+        if (fused)
+            CK(cudaFuncSetAttribute((const void *)k_bnc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin),
+               "configure kernels");
+    }
     auto grid = [&](const void *fn, int block, size_t smem) {
+        if (reuse) return 1;
         return std::max(1, std::min((P + block - 1) / block, resident_ctas(fn, dev, block, smem) * sms * gs));
     };
     const int g_isect = grid(f_isect, tb, stack_smem);
@@ -972,8 +1037,7 @@ lambda_status render_pass(lambda_ctx *ctx, const lambda_job *jobs, const std::ve
         return n;
     };
     auto clear = [&]() -> cudaError_t {
-        cudaError_t e = cudaMemsetAsync(ps.stats, 0, 8 * 8, stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(ps.error, 0, 16, stream);
+        cudaError_t e = cudaMemsetAsync(ps.stats, 0, kPassStatBytes, stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(ps.counts, 0, size_t(kQueues * (d_max + 2)) * 4, stream);
         return e;
     };
@@ -985,17 +1049,28 @@ lambda_status render_pass(lambda_ctx *ctx, const lambda_job *jobs, const std::ve
         return int32_t(std::min<int64_t>(completed_base + done, completed_total));
     };
     int launches = 0;
-    bool path_pass = false;
     std::vector<Progress> progress(completed ? size_t(s_max) : 0);
     // the surrogate flag changes nothing on a scene without thin films
     const bool film_surrogate = surrogate && (sc.families & (1u << 2)) != 0;
-    if (!film_surrogate && P <= tu.path_kernel_pixels) {
+    const bool path_pass = !film_surrogate && P <= tu.path_kernel_pixels;
+    if (!reuse && !prof) {
+        if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
+        ctx->graph_exec = nullptr;
+        ctx->plan_key.clear();
+    }
+    if (reuse) {
+        *ctx->progress_host = 0;
+        CK(cudaEventRecord(ctx->ev_start, stream), "event");
+        CK(cudaGraphLaunch(ctx->graph_exec, stream), "launch pass graph");
+        CK(cudaEventRecord(ctx->ev_stop, stream), "event");
+        launches = ctx->plan_launches;
+    } else if (path_pass) {
         // The pass as one persistent k_path launch (it seeds, traces and finishes
         // every pixel), captured with the counter clears into one graph.
         using PathKernel = void (*)(RenderParams, DeviceScene, PathState, int *, int *, int *);
         static const PathKernel path64[6] = {k_path<2, true>, k_path<4, true>, k_path<8, true>, k_path<2 | kCompressed, true>, k_path<4 | kCompressed, true>, k_path<8 | kCompressed, true>}, path32[6] = {k_path<2, false>, k_path<4, false>, k_path<8, false>, k_path<2 | kCompressed, false>, k_path<4 | kCompressed, false>, k_path<8 | kCompressed, false>};
         const PathKernel f_path = fp64 ? path64[li] : path32[li];
-        CK(cudaFuncSetAttribute((const void *)f_path, cudaFuncAttributeMaxDynamicSharedMemorySize, int(stack_smem)),
+        CK(cudaFuncSetAttribute((const void *)f_path, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin),
            "configure kernels");
         const int g_path = grid((const void *)f_path, tb, stack_smem);
         // counts[0]: the work counter (virtual pixels handed out); counts[1]: pixels done
@@ -1019,10 +1094,6 @@ lambda_status render_pass(lambda_ctx *ctx, const lambda_job *jobs, const std::ve
                 if (g) cudaGraphDestroy(g);
                 return ctx->cuda_fail(e != cudaSuccess ? e : ce, "capture path-kernel pass");
             }
-            if (ctx->graph_exec) {
-                cudaGraphExecDestroy(ctx->graph_exec);
-                ctx->graph_exec = nullptr;
-            }
             e = cudaGraphInstantiate(&ctx->graph_exec, g, 0);
             cudaGraphDestroy(g);
             if (e != cudaSuccess) return ctx->cuda_fail(e, "instantiate path-kernel pass");
@@ -1031,7 +1102,6 @@ lambda_status render_pass(lambda_ctx *ctx, const lambda_job *jobs, const std::ve
             CK(cudaEventRecord(ctx->ev_stop, stream), "event");
         }
         launches = 1;
-        path_pass = true;
     } else if (prof) {
         CK(clear(), "clear counters");
         CK(cudaEventRecord(ctx->ev_start, stream), "event");
@@ -1104,10 +1174,6 @@ lambda_status render_pass(lambda_ctx *ctx, const lambda_job *jobs, const std::ve
         if (ce != cudaSuccess) return fail(ce, "capture pass suffix");
         e = cudaGraphAddChildGraphNode(&n_post, g, &n_loop, 1, post);
         if (e != cudaSuccess) return fail(e, "build pass graph");
-        if (ctx->graph_exec) {
-            cudaGraphExecDestroy(ctx->graph_exec);
-            ctx->graph_exec = nullptr;
-        }
         e = cudaGraphInstantiate(&ctx->graph_exec, g, 0);
         cudaGraphDestroy(pre);
         cudaGraphDestroy(post);
@@ -1119,6 +1185,10 @@ lambda_status render_pass(lambda_ctx *ctx, const lambda_job *jobs, const std::ve
         CK(cudaGraphLaunch(ctx->graph_exec, stream), "launch pass graph");
         CK(cudaEventRecord(ctx->ev_stop, stream), "event");
         launches = 1 + s_max * wave_launches + 2;
+    }
+    if (!prof && !reuse) {
+        ctx->plan_key.assign(reinterpret_cast<const char *>(&key), reinterpret_cast<const char *>(&key) + sizeof(key));
+        ctx->plan_launches = launches;
     }
     if (completed && !prof) {
         // progress from the mapped host counter: the waves the graph has started, or
@@ -1145,11 +1215,12 @@ lambda_status render_pass(lambda_ctx *ctx, const lambda_job *jobs, const std::ve
                                stream),
                "copy image to host");
     }
-    unsigned long long stats[8] = {0};
-    int err[4] = {0};
-    CK(cudaMemcpyAsync(stats, ps.stats, sizeof(stats), cudaMemcpyDeviceToHost, stream), "read statistics");
-    CK(cudaMemcpyAsync(err, ps.error, sizeof(err), cudaMemcpyDeviceToHost, stream), "read flags");
+    CK(cudaMemcpyAsync(host_stats, ps.stats, kPassStatBytes, cudaMemcpyDeviceToHost, stream), "read statistics");
     CK(cudaStreamSynchronize(stream), "render");
+    unsigned long long stats[kPassStats];
+    int err[4];
+    std::memcpy(stats, host_stats, sizeof(stats));
+    std::memcpy(err, host_stats + sizeof(stats), sizeof(err));
     if (prof) CK(prof->collect(), "stage timing");
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop);
@@ -1626,25 +1697,32 @@ extern "C" lambda_status lambda_trace_shadow(lambda_ctx *ctx, const float *rays,
     if (!ctx->has_scene) return ctx->fail(LAMBDA_ERR_NO_SCENE, "no scene uploaded");
     if (n == 0) return LAMBDA_OK;
     // light ids are checked on the host: the kernel indexes instances/objects with them
-    std::vector<int32_t> hli(n), hlo(n);
-    if (is_device_pointer(light_instance)) CK(cudaMemcpy(hli.data(), light_instance, 4 * size_t(n), cudaMemcpyDeviceToHost), "read lights");
-    else std::memcpy(hli.data(), light_instance, 4 * size_t(n));
-    if (is_device_pointer(light_object)) CK(cudaMemcpy(hlo.data(), light_object, 4 * size_t(n), cudaMemcpyDeviceToHost), "read lights");
-    else std::memcpy(hlo.data(), light_object, 4 * size_t(n));
-    for (int k = 0; k < n; k++) {
-        const bool bg = hli[k] == -1 && hlo[k] == -1;
-        const bool ok = bg || (hli[k] >= 0 && hli[k] < ctx->dscene.num_instances && hlo[k] >= 0 && hlo[k] < ctx->dscene.num_objects);
-        if (!ok) return ctx->fail(LAMBDA_ERR_INVALID_ARGUMENT, "light id out of range");
-    }
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
+    std::vector<int32_t> hli, hlo;
+    auto on_host = [&](const int32_t *&p, std::vector<int32_t> &copy) {
+        if (!is_device_pointer(p)) return cudaSuccess;
+        copy.resize(size_t(n));
+        const cudaError_t e = cudaMemcpy(copy.data(), p, 4 * size_t(n), cudaMemcpyDeviceToHost);
+        p = copy.data();
+        return e;
+    };
+    CK(on_host(light_instance, hli), "read lights");
+    CK(on_host(light_object, hlo), "read lights");
+    unsigned bad = 0;
+    const unsigned ni = unsigned(ctx->dscene.num_instances), no = unsigned(ctx->dscene.num_objects);
+    for (int k = 0; k < n; k++) {
+        const unsigned i = unsigned(light_instance[k]), o = unsigned(light_object[k]);
+        bad |= unsigned(!((i < ni && o < no) || (i & o) == 0xFFFFFFFFu));
+    }
+    if (bad) return ctx->fail(LAMBDA_ERR_INVALID_ARGUMENT, "light id out of range");
     Staging sg{ctx, {}};
     CopyBack back;
     const float *dr;
     const int *dli, *dlo;
     int *docc;
     CK(sg.in(rays, size_t(n) * 6, &dr), "stage rays");
-    CK(sg.in(hli.data(), size_t(n), &dli), "stage lights");
-    CK(sg.in(hlo.data(), size_t(n), &dlo), "stage lights");
+    CK(sg.in(light_instance, size_t(n), &dli), "stage lights");
+    CK(sg.in(light_object, size_t(n), &dlo), "stage lights");
     CK(sg.out(out_occluded, size_t(n), &docc, back), "stage results");
     CK(ctx->rbuf.error.reserve(16), "allocate flags");
     int *err = ctx->rbuf.error.as<int>();

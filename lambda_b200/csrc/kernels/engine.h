@@ -46,6 +46,14 @@ struct StageProfiler {
     cudaError_t collect();
 };
 
+// Page-locked host memory, for small transfers that must not block or be staged.
+struct HostBuffer {
+    void *ptr = nullptr;
+    size_t bytes = 0;
+    cudaError_t reserve(size_t n);
+    void release();
+};
+
 struct SceneBuffers {
     DeviceBuffer nodes, prims, tri, instances, spectra, spectrum_flat, cspectra, cspectrum_flat, materials,
         material_props, scalar_tex, spectrum_tex, light_inst, light_obj, light_power, light_cdf, material_emission,
@@ -58,7 +66,7 @@ struct SceneBuffers {
 
 struct RenderBuffers {
     DeviceBuffer rng, film, lam, ray_o, ray_d, throughput, radiance, hit_id, sh_o, sh_d, sh_a, sh_light,
-        q0, q1, qs, qm0, qm1, qm2, counts, wave, stats, error, out, path_info, jobs, active, work, film_rows, film_out,
+        q0, q1, qs, qm0, qm1, qm2, counts, wave, stats, error, out, path_info, jobs, film_rows, film_out,
         film_in_domain;
 };
 
@@ -88,7 +96,14 @@ struct lambda_ctx {
 
     RenderBuffers rbuf;
     lambda_dev::PathState pstate{};
+    // The last pass's graph, its launch plan: every argument of its kernels and all that
+    // chose them (render_pass). A pass of the same shape launches it again; the images,
+    // cameras and seeds are read from the job table, which every call uploads.
     cudaGraphExec_t graph_exec = nullptr;
+    std::vector<char> plan_key;
+    int plan_launches = 0;
+    HostBuffer io;          // a pass's job table, statistics and flags
+    DeviceBuffer staging;   // host arrays of the query calls, kept between calls up to kStagingKeep
     lambda_render_stats stats{};
     lambda_stage_time stage_times[LAMBDA_NUM_STAGES]{};
     lambda_tuning tuning{256, 256, 1, 0, 4, LAMBDA_PATH_KERNEL_PIXELS, 0, 0, 0};  // launch shapes (max_pixels 0: no limit)
@@ -125,17 +140,35 @@ struct lambda_ctx {
                 &s.wide_code[0], &s.wide_code[1], &s.wide_code[2], &s.wide_planes[0], &s.wide_planes[1], &s.wide_planes[2], &s.wide_q[0], &s.wide_q[1], &s.wide_q[2],
                 &r.rng, &r.film, &r.lam, &r.ray_o, &r.ray_d, &r.throughput, &r.radiance, &r.hit_id,
                 &r.sh_o, &r.sh_d, &r.sh_a, &r.sh_light, &r.q0, &r.q1, &r.qs, &r.qm0, &r.qm1, &r.qm2, &r.counts, &r.wave,
-                &r.stats, &r.error, &r.out, &r.path_info, &r.jobs, &r.active, &r.work, &r.film_rows, &r.film_out,
-                &r.film_in_domain, &sbuf.weights_bf16, &sbuf.weights_f32};
+                &r.stats, &r.error, &r.out, &r.path_info, &r.jobs, &r.film_rows, &r.film_out,
+                &r.film_in_domain, &staging, &sbuf.weights_bf16, &sbuf.weights_f32};
     }
 };
 
-// Stages caller arrays (host or device) in and out of device memory.
+// Stages caller arrays (host or device) in and out of device memory. The copies lie in
+// the context's staging buffer, which keeps the size of its largest call up to
+// kStagingKeep bytes (a call blocks until its results are out, so no two share it); what
+// does not fit is allocated for the call. cudaMalloc and cudaFree of four arrays took
+// longer than 200,000 rays' traversal.
+constexpr size_t kStagingKeep = size_t(64) << 20;
 struct Staging {
     lambda_ctx *ctx;
     std::vector<void *> owned;
+    size_t used = 0;
     ~Staging() {
         for (void *p : owned) cudaFree(p);
+        if (used > ctx->staging.bytes && used <= kStagingKeep) ctx->staging.reserve(used);
+    }
+    cudaError_t take(size_t bytes, void **p) {
+        const size_t at = used, n = (std::max<size_t>(bytes, 16) + 255) / 256 * 256;
+        used += n;
+        if (at + n <= ctx->staging.bytes) {
+            *p = ctx->staging.as<char>() + at;
+            return cudaSuccess;
+        }
+        cudaError_t e = cudaMalloc(p, n);
+        if (e == cudaSuccess) owned.push_back(*p);
+        return e;
     }
     template <typename T>
     cudaError_t in(const T *src, size_t n, const T **dst) {
@@ -144,9 +177,8 @@ struct Staging {
             return cudaSuccess;
         }
         void *p = nullptr;
-        cudaError_t e = cudaMalloc(&p, std::max<size_t>(n * sizeof(T), 16));
+        cudaError_t e = take(n * sizeof(T), &p);
         if (e != cudaSuccess) return e;
-        owned.push_back(p);
         *dst = static_cast<const T *>(p);
         return cudaMemcpyAsync(p, src, n * sizeof(T), cudaMemcpyHostToDevice, ctx->stream);
     }
@@ -157,9 +189,8 @@ struct Staging {
             return cudaSuccess;
         }
         void *p = nullptr;
-        cudaError_t e = cudaMalloc(&p, std::max<size_t>(n * sizeof(T), 16));
+        cudaError_t e = take(n * sizeof(T), &p);
         if (e != cudaSuccess) return e;
-        owned.push_back(p);
         *dst = static_cast<T *>(p);
         back.push_back({user, {p, n * sizeof(T)}});
         return cudaSuccess;

@@ -1180,19 +1180,21 @@ extern "C" lambda_status lambda_surrogate_train(lambda_ctx *ctx, const lambda_tr
     const int audit_n = 1 << 18;
     DeviceBuffer x, y, ax, ay, params, grad, m, v, loss, aout, partial;
     const int slots = int(std::min<int64_t>(std::min<int64_t>(d.batch, N) / kTrainRows + 1, ctx->sm_count));
-    // one allocation for the whole run, cut into 256-byte aligned parts: a cudaMalloc and
-    // its cudaFree take as long as several training steps
-    DeviceBuffer arena;
+    // one allocation for the whole run, cut into 256-byte aligned parts, from the
+    // context's staging memory where that keeps it: a cudaMalloc and its cudaFree take as
+    // long as tens of training steps
+    Staging sg{ctx, {}};
+    void *arena = nullptr;
     const std::pair<DeviceBuffer *, size_t> parts[] = {
         {&x, size_t(N) * kRowStride * 4}, {&y, size_t(N) * 16}, {&ax, size_t(audit_n) * kRowStride * 4},
         {&ay, size_t(audit_n) * 16}, {&aout, size_t(audit_n) * 16}, {&partial, 2 * kAuditBlocks * sizeof(double)},
         {&params, kParams * 4}, {&grad, size_t(slots) * kParams * 4}, {&m, kParams * 4}, {&v, kParams * 4}, {&loss, 64}};
     size_t arena_bytes = 0;
     for (const auto &q : parts) arena_bytes += (q.second + 255) / 256 * 256;
-    CK(arena.reserve(arena_bytes), "allocate training set");
+    CK(sg.take(arena_bytes, &arena), "allocate training set");
     size_t off = 0;
     for (const auto &q : parts) {
-        *q.first = DeviceBuffer{arena.as<char>() + off, q.second};
+        *q.first = DeviceBuffer{static_cast<char *>(arena) + off, q.second};
         off += (q.second + 255) / 256 * 256;
     }
     cudaEvent_t e0, e1, e2;
@@ -1276,7 +1278,6 @@ extern "C" lambda_status lambda_surrogate_train(lambda_ctx *ctx, const lambda_tr
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaEventDestroy(e2);
-    arena.release();
     return LAMBDA_OK;
 }
 
