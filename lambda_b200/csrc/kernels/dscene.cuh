@@ -222,12 +222,16 @@ struct ShadePoint {
     float u, v;
 };
 
-__device__ __forceinline__ float scalar_texture(const DeviceScene &s, int t, f3 p) {
-    const float4 x = __ldg(&s.scalar_tex[t]);
+// A scalar texture given its record (DeviceScene::scalar_tex).
+__device__ __forceinline__ float scalar_record(const DeviceScene &s, const float4 &x, f3 p) {
     const int type = __float_as_int(x.x);
     if (type == 0) return x.y;                                            // constant
     if (type == 1) return x.y + (x.z - x.y) * perlin_noise(s, p * x.w);   // perlin
     return x.y + (x.z - x.y) * worley_noise(s, p * x.w);                  // worley
+}
+
+__device__ __forceinline__ float scalar_texture(const DeviceScene &s, int t, f3 p) {
+    return scalar_record(s, __ldg(&s.scalar_tex[t]), p);
 }
 
 __device__ __forceinline__ float spectrum_texture(const DeviceScene &s, int t, const ShadePoint &sp, float lambda) {
@@ -242,9 +246,19 @@ __device__ __forceinline__ float spectrum_texture(const DeviceScene &s, int t, c
     return scalar_texture(s, x.y, sp.point);
 }
 
-// A spectrum texture at the four hero wavelengths; a texture that does not
-// depend on the wavelength (scalar) is evaluated once.
+// A spectrum texture at the four hero wavelengths. Its record answers for a constant
+// spectrum whose bins are all equal (a is the value) and a checker of two such (a, b),
+// the values the lookups below would return; a texture that does not depend on the
+// wavelength (scalar) is evaluated once.
 __device__ __forceinline__ s4 spectrum_texture4(const DeviceScene &s, int t, const ShadePoint &sp, const s4 &lam) {
+    const float4 rec = __ldg(&s.tex_record[t]);
+    const int kind = __float_as_int(rec.x);
+    if (kind == kTexFlat) return s4_fill(rec.y);
+    if (kind == kTexFlatChecker) {
+        const int cx = int(floorf(sp.u / rec.w));
+        const int cy = int(floorf(sp.v / rec.w));
+        return s4_fill((cx + cy) % 2 == 0 ? rec.y : rec.z);
+    }
     const int4 x = __ldg(&s.spectrum_tex[t]);
     if (x.x == 2) return s4_fill(scalar_texture(s, x.y, sp.point));
     s4 r;
@@ -1072,24 +1086,27 @@ __device__ __forceinline__ float prim_area(const Prim &p) {
 
 enum : int { kLambertian = 0, kMirror = 1, kDielectric = 2, kEmissive = 3, kThinFilm = 4 };
 
-// CIE 1931 lookup with linear interpolation (utils.h:195-203) and the
-// spectrum -> XYZ -> linear sRGB conversion (utils.h:212-231).
-__device__ __forceinline__ float xyz31(const DeviceScene &s, float lambda, int i) {
-    const int lo = int(lambda);
-    if (lo == 830) return s.cie[(lo - 360) * 3 + i];
-    const int hi = lo + 1;
-    return (float(hi) - lambda) * s.cie[(lo - 360) * 3 + i] + (lambda - float(lo)) * s.cie[(hi - 360) * 3 + i];
-}
-
+// The spectrum -> XYZ -> linear sRGB conversion (utils.h:212-231) with the CIE 1931 lookup
+// interpolated linearly (utils.h:195-203); a bin's three values come in one load.
 __device__ __forceinline__ f3 spectrum_to_rgb(const DeviceScene &s, const s4 &L, const s4 &lam, float range) {
     float x = 0, y = 0, z = 0;
     const float w = range / kHero;
     for (int i = 0; i < kHero; i++) {
         const float l = lam.v[i];
         const float r = L.v[i];
-        x += xyz31(s, l, 0) * r * w;
-        y += xyz31(s, l, 1) * r * w;
-        z += xyz31(s, l, 2) * r * w;
+        const int lo = int(l);
+        f3 c;
+        const float4 a = __ldg(&s.cie[lo - 360]);
+        if (lo == 830) {
+            c = mk(a.x, a.y, a.z);
+        } else {
+            const float4 b = __ldg(&s.cie[lo - 359]);
+            const float wa = float(lo + 1) - l, wb = l - float(lo);
+            c = mk(wa * a.x + wb * b.x, wa * a.y + wb * b.y, wa * a.z + wb * b.z);
+        }
+        x += c.x * r * w;
+        y += c.y * r * w;
+        z += c.z * r * w;
     }
     x /= 106.856895f;
     y /= 106.856895f;

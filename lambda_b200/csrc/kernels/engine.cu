@@ -476,9 +476,9 @@ extern "C" lambda_status lambda_scene_upload(lambda_ctx *ctx, const lambda_scene
         run += d.light_powers[i];
         cdf[i] = run;
     }
-    std::vector<float> cie(LAMBDA_CIE_BINS * 3);
+    std::vector<float4> cie(LAMBDA_CIE_BINS);
     for (int i = 0; i < LAMBDA_CIE_BINS; i++)
-        for (int k = 0; k < 3; k++) cie[3 * i + k] = float(kCieXyz1931[i][k]);
+        cie[i] = make_float4(float(kCieXyz1931[i][0]), float(kCieXyz1931[i][1]), float(kCieXyz1931[i][2]), 0.0f);
     std::vector<float4> worley;
     int3 wlo, wdim;
     build_worley_table(d, worley, wlo, wdim);
@@ -502,6 +502,29 @@ extern "C" lambda_status lambda_scene_upload(lambda_ctx *ctx, const lambda_scene
         if (ok) film_flat[size_t(i)] = make_float4(v[0], v[1], v[2], 1.0f);
     }
 
+    auto bits = [](int v) {
+        float f;
+        std::memcpy(&f, &v, 4);
+        return f;
+    };
+    std::vector<float4> tex_record(d.num_spectrum_textures);
+    for (int i = 0; i < d.num_spectrum_textures; i++) {
+        const lambda_spectrum_texture &t = d.spectrum_textures[i];
+        tex_record[i] = make_float4(bits(kTexGeneral), 0, 0, 0);
+        auto value = [&](int k) { return d.spectra[size_t(k) * LAMBDA_CIE_BINS]; };
+        if (t.type == LAMBDA_SPECTRUM_CONSTANT && flat[t.value1])
+            tex_record[i] = make_float4(bits(kTexFlat), value(t.value1), 0, 0);
+        else if (t.type == LAMBDA_SPECTRUM_CHECKER && flat[t.value1] && flat[t.value2])
+            tex_record[i] = make_float4(bits(kTexFlatChecker), value(t.value1), value(t.value2), t.scale);
+    }
+    std::vector<float4> film_layer(size_t(std::max(d.num_materials, 1)), make_float4(0, 0, 0, 0));
+    for (int i = 0; i < d.num_materials; i++)
+        if (d.materials[i].type == LAMBDA_MATERIAL_THINFILM && d.materials[i].p[0] == 1)
+            film_layer[size_t(i)] = stex[d.material_properties[d.materials[i].p[2]]];
+    std::vector<float4> light_record(d.num_lights);
+    for (int i = 0; i < d.num_lights; i++)
+        light_record[i] = make_float4(cdf[i], d.light_powers[i], bits(d.light_instances[i]), bits(d.light_objects[i]));
+
     CK(b.nodes.upload(nodes.data(), nodes.size() * sizeof(float4), s), "upload nodes");
     CK(b.prims.upload(prims.data(), prims.size() * sizeof(float4), s), "upload objects");
     CK(b.tri.upload(tri.data(), tri.size() * sizeof(float4), s), "upload triangles");
@@ -522,7 +545,10 @@ extern "C" lambda_status lambda_scene_upload(lambda_ctx *ctx, const lambda_scene
     CK(b.material_emission.upload(emission.data(), emission.size() * sizeof(float), s), "upload materials");
     CK(b.material_uv.upload(muv.data(), muv.size(), s), "upload materials");
     CK(b.film_flat.upload(film_flat.data(), film_flat.size() * sizeof(float4), s), "upload materials");
-    CK(b.cie.upload(cie.data(), cie.size() * sizeof(float), s), "upload CIE table");
+    CK(b.tex_record.upload(tex_record.data(), tex_record.size() * sizeof(float4), s), "upload textures");
+    CK(b.film_layer.upload(film_layer.data(), film_layer.size() * sizeof(float4), s), "upload materials");
+    CK(b.light_record.upload(light_record.data(), light_record.size() * sizeof(float4), s), "upload lights");
+    CK(b.cie.upload(cie.data(), cie.size() * sizeof(float4), s), "upload CIE table");
     CK(b.perm.upload(kPerlinPermutation, sizeof(kPerlinPermutation), s), "upload permutation");
     CK(b.worley.upload(worley.data(), worley.size() * sizeof(float4), s), "upload Worley lattice");
     for (int k = 0; k < 3; k++) {
@@ -604,9 +630,12 @@ extern "C" lambda_status lambda_scene_upload(lambda_ctx *ctx, const lambda_scene
     ds.material_emission = b.material_emission.as<float>();
     ds.material_uv = b.material_uv.as<uint8_t>();
     ds.film_flat = b.film_flat.as<float4>();
+    ds.tex_record = b.tex_record.as<float4>();
+    ds.film_layer = b.film_layer.as<float4>();
+    ds.light_record = b.light_record.as<float4>();
     ds.instance_flags = b.instance_flags.as<uint32_t>();
     ds.families = families;
-    ds.cie = b.cie.as<float>();
+    ds.cie = b.cie.as<float4>();
     ds.perm = b.perm.as<int>();
     ds.worley_cells = b.worley.as<float4>();
     ds.worley_lo = wlo;

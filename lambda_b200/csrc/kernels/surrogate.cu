@@ -852,7 +852,7 @@ __global__ void __launch_bounds__(256) k_film_encode(int bounce, RenderParams rp
         const int p = q[idx];
         const ShadeIn s = load_shade(ps, sc, p);
         bool ok = s.m.y == 1;
-        const float d = ok ? scalar_texture(sc, sc.material_props[s.m.w], s.sp.point) : 0.0f;
+        const float d = ok ? scalar_record(sc, __ldg(&sc.film_layer[s.mat]), s.sp.point) : 0.0f;
         const float cos_in = dot(s.nrm, -s.d);
         ok = ok && d >= fs.d_lo && d <= fs.d_hi;
         float e[kHero][kIn];

@@ -49,6 +49,36 @@ __device__ __forceinline__ int warp_push(int *counter, bool want) {
     return want ? base + __popc(mask & ((1u << lane) - 1u)) : -1;
 }
 
+// Pushes to N queues at once: lane f adds for counter[f], so the N atomics are one
+// instruction and cost one round trip. Must be reached by all 32 lanes; slot[f] is
+// valid where want[f].
+template <int N>
+__device__ __forceinline__ void warp_push_n(int *const (&counter)[N], const bool (&want)[N], int (&slot)[N]) {
+    const int lane = threadIdx.x & 31;
+    unsigned mask[N], any = 0, mine = 0;
+    int *at = counter[0];
+#pragma unroll
+    for (int f = 0; f < N; f++) {
+        mask[f] = __ballot_sync(0xffffffffu, want[f]);
+        any |= mask[f];
+        if (lane == f) {
+            mine = mask[f];
+            at = counter[f];
+        }
+    }
+    if (any == 0) return;
+    int base = 0;
+    if (mine) base = atomicAdd(at, __popc(mine));
+#pragma unroll
+    for (int f = 0; f < N; f++) slot[f] = __shfl_sync(0xffffffffu, base, f) + __popc(mask[f] & ((1u << lane) - 1u));
+}
+
+// Entry idx of a queue of at most rp.num_pixels entries, read without waiting for the
+// queue's size (an entry past it is stale and not used).
+__device__ __forceinline__ int queue_entry(const RenderParams &rp, const int *q, int idx) {
+    return idx < rp.num_pixels ? q[idx] : 0;
+}
+
 __device__ __forceinline__ s4 hero_wavelengths(const Job &job, float lambda0) {
     s4 l;
     for (int k = 0; k < kHero; k++) {
@@ -145,14 +175,15 @@ LAMBDA_KERNEL void k_wave_prologue(int depth, PathState ps, cudaGraphConditional
 // the material it was absorbed at) and before the first one.
 __device__ __forceinline__ s4 ended_emission(const DeviceScene &sc, const PathState &ps, int p, const s4 &lam) {
     const int4 id = ps.hit_id[p];
+    // read beside the hit id, not after it: most samples end at a miss or an emitter
+    const float4 o4 = ps.ray_o[p], d4 = ps.ray_d[p];
+    const s4 T = from_f4(ps.throughput[p]);
     if (id.y == kNoHit) return s4_fill(0);
     const bool lights = sc.total_light_power > 0;
     int4 m = make_int4(kEmissive, 0, 0, 0);
     if (id.y != kMissed) m = __ldg(&sc.materials[id.x]);
     if (m.x != kEmissive) return s4_fill(0);
-    const float4 o4 = ps.ray_o[p], d4 = ps.ray_d[p];
     const f3 o = mk(o4.x, o4.y, o4.z), d = mk(d4.x, d4.y, d4.z);
-    const s4 T = from_f4(ps.throughput[p]);
     const bool specular = d4.w != 0.0f;
     const float prev_pdf = o4.w;
     if (id.y == kMissed) {
@@ -290,17 +321,18 @@ LAMBDA_KERNEL void __launch_bounds__(256, 4) k_intersect(int bounce, RenderParam
     const int n = ps.counts[queue_slot(bounce, kQActive)];
     const int *q = ps.queue[bounce & 1];
     const int stride = gridDim.x * blockDim.x;
+    int next = queue_entry(rp, q, blockIdx.x * blockDim.x + threadIdx.x);
     for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
-        const int idx = base + threadIdx.x;
-        int p = 0, family = -1;
-        if (idx < n) {
-            p = q[idx];
-            family = trace_path<K>(sc, ps, p, st_a, st_b);
-        }
-        for (int f = 0; f < 3; f++) {
-            const int slot = warp_push(&ps.counts[queue_slot(bounce, kQLambert + f)], family == f);
-            if (family == f) ps.mat_queue[f][slot] = p;
-        }
+        const int idx = base + threadIdx.x, p = next;
+        next = queue_entry(rp, q, idx + stride);
+        int family = -1;
+        if (idx < n) family = trace_path<K>(sc, ps, p, st_a, st_b);
+        int *const at = &ps.counts[queue_slot(bounce, kQLambert)];
+        int slot[3];
+        warp_push_n<3>({at, at + 1, at + 2}, {family == 0, family == 1, family == 2}, slot);
+        if (family == 0) ps.mat_queue[0][slot[0]] = p;
+        if (family == 1) ps.mat_queue[1][slot[1]] = p;
+        if (family == 2) ps.mat_queue[2][slot[2]] = p;
     }
 }
 
@@ -507,21 +539,24 @@ __device__ __forceinline__ bool finish_scatter(const PathState &ps, const ShadeI
 // NEE ray in the path state and setting `nee`, then cosine-weighted scatter
 // (material.h:151-172). Returns whether the path continues.
 __device__ __forceinline__ bool lambert_path(const DeviceScene &sc, const PathState &ps, int p, int bounce, bool &nee) {
+    const float4 first_light = __ldg(sc.light_record);
     const ShadeIn s = load_shade(ps, sc, p);
     Rng rng = path_rng(ps, p);
     const s4 albedo = spectrum_texture4(sc, s.m.y, s.sp, s.lam);
     if (sc.total_light_power > 0) {
         const float target = sc.total_light_power * rng.next();
-        int li = sc.light_inst[0], lo = sc.light_obj[0];
-        float lp = sc.light_power[0];
-        for (int j = 0; j < sc.num_lights; j++) {
-            if (sc.light_cdf[j] >= target) {
-                li = sc.light_inst[j];
-                lo = sc.light_obj[j];
-                lp = sc.light_power[j];
-                break;
+        float4 light = first_light;  // also when no running sum reaches the target
+        if (!(light.x >= target)) {
+            for (int j = 1; j < sc.num_lights; j++) {
+                const float4 l = __ldg(&sc.light_record[j]);
+                if (l.x >= target) {
+                    light = l;
+                    break;
+                }
             }
         }
+        const int li = __float_as_int(light.z), lo = __float_as_int(light.w);
+        const float lp = light.y;
         f3 ldir;
         float lpdf;
         if (li != -1) {
@@ -571,18 +606,17 @@ LAMBDA_KERNEL void __launch_bounds__(256, 3) k_shade_lambert(int bounce, RenderP
     const int *q = ps.mat_queue[0];
     int *q_next = ps.queue[(bounce + 1) & 1];
     const int stride = gridDim.x * blockDim.x;
+    int next = queue_entry(rp, q, blockIdx.x * blockDim.x + threadIdx.x);
     for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
-        const int idx = base + threadIdx.x;
+        const int idx = base + threadIdx.x, p = next;
+        next = queue_entry(rp, q, idx + stride);
         bool alive = false, nee = false;
-        int p = 0;
-        if (idx < n) {
-            p = q[idx];
-            alive = lambert_path(sc, ps, p, bounce, nee);
-        }
-        const int slot = warp_push(&ps.counts[queue_slot(bounce + 1, kQActive)], alive);
-        if (alive) q_next[slot] = p;
-        const int sslot = warp_push(&ps.counts[queue_slot(bounce, kQShadow)], nee);
-        if (nee) ps.shadow_queue[sslot] = p;
+        if (idx < n) alive = lambert_path(sc, ps, p, bounce, nee);
+        int slot[2];
+        warp_push_n<2>({&ps.counts[queue_slot(bounce + 1, kQActive)], &ps.counts[queue_slot(bounce, kQShadow)]}, {alive, nee},
+                       slot);
+        if (alive) q_next[slot[0]] = p;
+        if (nee) ps.shadow_queue[slot[1]] = p;
     }
 }
 
@@ -632,14 +666,12 @@ LAMBDA_KERNEL void __launch_bounds__(256) k_shade_specular(int bounce, RenderPar
     const int *q = ps.mat_queue[1];
     int *q_next = ps.queue[(bounce + 1) & 1];
     const int stride = gridDim.x * blockDim.x;
+    int next = queue_entry(rp, q, blockIdx.x * blockDim.x + threadIdx.x);
     for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
-        const int idx = base + threadIdx.x;
+        const int idx = base + threadIdx.x, p = next;
+        next = queue_entry(rp, q, idx + stride);
         bool alive = false;
-        int p = 0;
-        if (idx < n) {
-            p = q[idx];
-            alive = specular_path(sc, ps, p, bounce);
-        }
+        if (idx < n) alive = specular_path(sc, ps, p, bounce);
         const int slot = warp_push(&ps.counts[queue_slot(bounce + 1, kQActive)], alive);
         if (alive) q_next[slot] = p;
     }
@@ -782,6 +814,10 @@ __device__ __forceinline__ void thin_film_scatter(const DeviceScene &sc, const S
 // per hit (the reference evaluates them once per wavelength at the same point).
 __device__ __forceinline__ void thin_film_thickness(const DeviceScene &sc, const ShadeIn &s, float *thick) {
     const int L = s.m.y < kMaxFilmLayers ? s.m.y : kMaxFilmLayers;
+    if (L == 1) {
+        thick[0] = scalar_record(sc, __ldg(&sc.film_layer[s.mat]), s.sp.point);
+        return;
+    }
     for (int k = 0; k < L; k++) thick[k] = scalar_texture(sc, sc.material_props[s.m.w + k], s.sp.point);
 }
 
