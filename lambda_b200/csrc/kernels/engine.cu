@@ -414,6 +414,15 @@ extern "C" lambda_status lambda_scene_upload(lambda_ctx *ctx, const lambda_scene
             tri[4 * i + 3] = make_float4(g[24], g[25], g[26], 0);
         } else {
             for (int k = 0; k < 4; k++) tri[4 * i + k] = make_float4(0, 0, 0, 0);
+            if (o.type == LAMBDA_OBJECT_QUAD) {
+                // as the device forms them (no contraction, correctly rounded root and quotients)
+                const float nsq = g[9] * g[9] + g[10] * g[10] + g[11] * g[11], l = std::sqrt(nsq);
+                const float n[3] = {g[9] / l, g[10] / l, g[11] / l};
+                tri[4 * i] = make_float4(n[0], n[1], n[2], nsq);
+                const float w[3] = {n[0] + 0.0f, n[1] + 0.0f, n[2] + 0.0f};  // to_world of an identity instance
+                const float lw = std::sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
+                tri[4 * i + 1] = make_float4(w[0] / lw, w[1] / lw, w[2] / lw, 0);
+            }
         }
     }
     std::vector<float4> inst(9 * size_t(d.num_instances));
