@@ -42,7 +42,10 @@ lambda_status lambda_ctx::fail(lambda_status s, const std::string &msg) {
     return s;
 }
 
+// Reports a failed runtime call. The error also stays in cudaGetLastError, where the check
+// after a later call's launch would take it for that launch's, so it is cleared here.
 lambda_status lambda_ctx::cuda_fail(cudaError_t e, const char *what) {
+    cudaGetLastError();
     last_error = std::string(what) + " (" + cudaGetErrorString(e) + ")";
     return e == cudaErrorMemoryAllocation ? LAMBDA_ERR_OUT_OF_MEMORY : LAMBDA_ERR_CUDA;
 }

@@ -157,7 +157,8 @@ struct Staging {
     size_t used = 0;
     ~Staging() {
         for (void *p : owned) cudaFree(p);
-        if (used > ctx->staging.bytes && used <= kStagingKeep) ctx->staging.reserve(used);
+        if (used > ctx->staging.bytes && used <= kStagingKeep && ctx->staging.reserve(used) != cudaSuccess)
+            cudaGetLastError();  // the call has its results; the next one allocates again
     }
     cudaError_t take(size_t bytes, void **p) {
         const size_t at = used, n = (std::max<size_t>(bytes, 16) + 255) / 256 * 256;
