@@ -1694,9 +1694,34 @@ cudaError_t launch_query(lambda_ctx *ctx, void (*const *fns)(DeviceScene, A...),
 
 }  // namespace
 
-lambda_status finish_staging(lambda_ctx *ctx, CopyBack &back) {
-    for (auto &b : back)
-        CK(cudaMemcpyAsync(b.first, b.second.first, b.second.second, cudaMemcpyDeviceToHost, ctx->stream), "copy results");
+cudaError_t Staging::begin() {
+    if (parts.empty()) return cudaSuccess;
+    cudaError_t e;
+    if (total <= kStagingKeep) {
+        e = ctx->staging.reserve(total);
+        base = ctx->staging.as<char>();
+    } else {
+        e = cudaMalloc(&own, total);
+        if (e == cudaErrorMemoryAllocation && ctx->staging.ptr) {  // the kept memory may be what is missing
+            cudaGetLastError();
+            ctx->staging.release();
+            e = cudaMalloc(&own, total);
+        }
+        if (e != cudaSuccess) own = nullptr;
+        base = static_cast<char *>(own);
+    }
+    for (const Part &p : parts) {
+        if (e != cudaSuccess) return e;
+        void *at = base + p.at;
+        std::memcpy(p.dst, &at, sizeof(at));
+        if (p.src) e = cudaMemcpyAsync(at, p.src, p.bytes, cudaMemcpyHostToDevice, ctx->stream);
+    }
+    return e;
+}
+
+lambda_status Staging::finish() {
+    for (const Part &p : parts)
+        if (p.user) CK(cudaMemcpyAsync(p.user, base + p.at, p.bytes, cudaMemcpyDeviceToHost, ctx->stream), "copy results");
     CK(cudaStreamSynchronize(ctx->stream), "query");
     return LAMBDA_OK;
 }
@@ -1707,15 +1732,15 @@ extern "C" lambda_status lambda_trace_closest(lambda_ctx *ctx, const float *rays
     if (!ctx->has_scene) return ctx->fail(LAMBDA_ERR_NO_SCENE, "no scene uploaded");
     if (n == 0) return LAMBDA_OK;
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
-    Staging sg{ctx, {}};
-    CopyBack back;
+    Staging sg(ctx);
     const float *dr;
     int *di, *dobj;
     float *dt;
-    CK(sg.in(rays, size_t(n) * 6, &dr), "stage rays");
-    CK(sg.out(out_instance, size_t(n), &di, back), "stage results");
-    CK(sg.out(out_object, size_t(n), &dobj, back), "stage results");
-    CK(sg.out(out_t, size_t(n), &dt, back), "stage results");
+    sg.in(rays, size_t(n) * 6, &dr);
+    sg.out(out_instance, size_t(n), &di);
+    sg.out(out_object, size_t(n), &dobj);
+    sg.out(out_t, size_t(n), &dt);
+    CK(sg.begin(), "stage rays");
     CK(ctx->rbuf.error.reserve(16), "allocate flags");
     int *err = ctx->rbuf.error.as<int>();
     CK(cudaMemsetAsync(err, 0, 16, ctx->stream), "clear flags");
@@ -1725,7 +1750,7 @@ extern "C" lambda_status lambda_trace_closest(lambda_ctx *ctx, const float *rays
     CK(cudaGetLastError(), "launch trace");
     int herr = 0;
     CK(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, ctx->stream), "read flags");
-    lambda_status s = finish_staging(ctx, back);
+    lambda_status s = sg.finish();
     if (s != LAMBDA_OK) return s;
     if (herr & 1) return ctx->fail(LAMBDA_ERR_QUEUE_OVERFLOW, "BVH traversal stack overflow");
     return LAMBDA_OK;
@@ -1756,15 +1781,15 @@ extern "C" lambda_status lambda_trace_shadow(lambda_ctx *ctx, const float *rays,
         bad |= unsigned(!((i < ni && o < no) || (i & o) == 0xFFFFFFFFu));
     }
     if (bad) return ctx->fail(LAMBDA_ERR_INVALID_ARGUMENT, "light id out of range");
-    Staging sg{ctx, {}};
-    CopyBack back;
+    Staging sg(ctx);
     const float *dr;
     const int *dli, *dlo;
     int *docc;
-    CK(sg.in(rays, size_t(n) * 6, &dr), "stage rays");
-    CK(sg.in(light_instance, size_t(n), &dli), "stage lights");
-    CK(sg.in(light_object, size_t(n), &dlo), "stage lights");
-    CK(sg.out(out_occluded, size_t(n), &docc, back), "stage results");
+    sg.in(rays, size_t(n) * 6, &dr);
+    sg.in(light_instance, size_t(n), &dli);
+    sg.in(light_object, size_t(n), &dlo);
+    sg.out(out_occluded, size_t(n), &docc);
+    CK(sg.begin(), "stage rays");
     CK(ctx->rbuf.error.reserve(16), "allocate flags");
     int *err = ctx->rbuf.error.as<int>();
     CK(cudaMemsetAsync(err, 0, 16, ctx->stream), "clear flags");
@@ -1776,7 +1801,7 @@ extern "C" lambda_status lambda_trace_shadow(lambda_ctx *ctx, const float *rays,
     CK(cudaGetLastError(), "launch trace");
     int herr = 0;
     CK(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, ctx->stream), "read flags");
-    lambda_status s = finish_staging(ctx, back);
+    lambda_status s = sg.finish();
     if (s != LAMBDA_OK) return s;
     if (herr & 1) return ctx->fail(LAMBDA_ERR_QUEUE_OVERFLOW, "BVH traversal stack overflow");
     return LAMBDA_OK;
@@ -1853,12 +1878,12 @@ lambda_status film_query(lambda_ctx *ctx, const lambda_film_query *q, int32_t n,
     if (!ctx || n < 0 || (n > 0 && (!q || !out))) return LAMBDA_ERR_INVALID_ARGUMENT;
     if (n == 0) return LAMBDA_OK;
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
-    Staging sg{ctx, {}};
-    CopyBack back;
+    Staging sg(ctx);
     const lambda_film_query *dq;
     R *dout;
-    CK(sg.in(q, size_t(n), &dq), "stage queries");
-    CK(sg.out(out, size_t(n) * 4, &dout, back), "stage results");
+    sg.in(q, size_t(n), &dq);
+    sg.out(out, size_t(n) * 4, &dout);
+    CK(sg.begin(), "stage queries");
     const bool aligned = ((reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dout)) & 15u) == 0;
     if constexpr (sizeof(R) == 4) {
         if (aligned && n >= kFilmQuery4Min)
@@ -1869,7 +1894,7 @@ lambda_status film_query(lambda_ctx *ctx, const lambda_film_query *q, int32_t n,
         k_film_query<R><<<(n + 127) / 128, 128, 0, ctx->stream>>>(dq, n, dout);
     }
     CK(cudaGetLastError(), "launch thin-film query");
-    return finish_staging(ctx, back);
+    return sg.finish();
 }
 
 }  // namespace

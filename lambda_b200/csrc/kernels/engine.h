@@ -145,61 +145,53 @@ struct lambda_ctx {
     }
 };
 
-// Stages caller arrays (host or device) in and out of device memory. The copies lie in
-// the context's staging buffer, which keeps the size of its largest call up to
-// kStagingKeep bytes (a call blocks until its results are out, so no two share it); what
-// does not fit is allocated for the call. cudaMalloc and cudaFree of four arrays took
-// longer than 200,000 rays' traversal.
+// Stages caller arrays (host or device) in and out of device memory: a call names its
+// arrays (in, out, scratch), begin() finds room for all of them at once and copies the
+// inputs in, finish() copies the results out and waits. The copies lie in the context's
+// staging buffer, which keeps the size of its largest call up to kStagingKeep bytes (a
+// call blocks until its results are out, so no two share it); a larger call has one
+// allocation of its own. cudaMalloc and cudaFree of four arrays took longer than 200,000
+// rays' traversal.
 constexpr size_t kStagingKeep = size_t(64) << 20;
-struct Staging {
-    lambda_ctx *ctx;
-    std::vector<void *> owned;
-    size_t used = 0;
+class Staging {
+public:
+    explicit Staging(lambda_ctx *c) : ctx(c) {}
     ~Staging() {
-        for (void *p : owned) cudaFree(p);
-        if (used > ctx->staging.bytes && used <= kStagingKeep && ctx->staging.reserve(used) != cudaSuccess)
-            cudaGetLastError();  // the call has its results; the next one allocates again
+        if (own) cudaFree(own);
     }
-    cudaError_t take(size_t bytes, void **p) {
-        const size_t at = used, n = (std::max<size_t>(bytes, 16) + 255) / 256 * 256;
-        used += n;
-        if (at + n <= ctx->staging.bytes) {
-            *p = ctx->staging.as<char>() + at;
-            return cudaSuccess;
-        }
-        cudaError_t e = cudaMalloc(p, n);
-        if (e == cudaSuccess) owned.push_back(*p);
-        return e;
+    Staging(const Staging &) = delete;
+    Staging &operator=(const Staging &) = delete;
+
+    // *dst (set by begin() where src is host memory): n values on the device
+    template <typename T>
+    void in(const T *src, size_t n, const T **dst) {
+        if (is_device_pointer(src)) *dst = src;
+        else place(dst, src, nullptr, n * sizeof(T));
     }
     template <typename T>
-    cudaError_t in(const T *src, size_t n, const T **dst) {
-        if (is_device_pointer(src)) {
-            *dst = src;
-            return cudaSuccess;
-        }
-        void *p = nullptr;
-        cudaError_t e = take(n * sizeof(T), &p);
-        if (e != cudaSuccess) return e;
-        *dst = static_cast<const T *>(p);
-        return cudaMemcpyAsync(p, src, n * sizeof(T), cudaMemcpyHostToDevice, ctx->stream);
+    void out(T *user, size_t n, T **dst) {
+        if (is_device_pointer(user)) *dst = user;
+        else place(dst, nullptr, user, n * sizeof(T));
     }
-    template <typename T>
-    cudaError_t out(T *user, size_t n, T **dst, std::vector<std::pair<void *, std::pair<void *, size_t>>> &back) {
-        if (is_device_pointer(user)) {
-            *dst = user;
-            return cudaSuccess;
-        }
-        void *p = nullptr;
-        cudaError_t e = take(n * sizeof(T), &p);
-        if (e != cudaSuccess) return e;
-        *dst = static_cast<T *>(p);
-        back.push_back({user, {p, n * sizeof(T)}});
-        return cudaSuccess;
+    void scratch(size_t bytes, void **dst) { place(dst, nullptr, nullptr, bytes); }
+
+    cudaError_t begin();
+    lambda_status finish();
+
+private:
+    struct Part {
+        void *dst;  // the pointer variable to set
+        const void *src;
+        void *user;
+        size_t bytes, at;
+    };
+    void place(void *dst, const void *src, void *user, size_t bytes) {
+        parts.push_back(Part{dst, src, user, bytes, total});
+        total += (std::max<size_t>(bytes, 16) + 255) / 256 * 256;
     }
+    lambda_ctx *ctx;
+    std::vector<Part> parts;
+    size_t total = 0;
+    char *base = nullptr;
+    void *own = nullptr;
 };
-
-using CopyBack = std::vector<std::pair<void *, std::pair<void *, size_t>>>;
-
-// Copies staged results back to the caller's host arrays and waits for the stream.
-lambda_status finish_staging(lambda_ctx *ctx, CopyBack &back);
-

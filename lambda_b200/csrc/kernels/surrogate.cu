@@ -1134,15 +1134,15 @@ extern "C" lambda_status lambda_surrogate_eval(lambda_ctx *ctx, const lambda_fil
     if (!ctx->has_surrogate) return ctx->fail(LAMBDA_ERR_INVALID_ARGUMENT, "no surrogate installed");
     if (n == 0) return LAMBDA_OK;
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
-    Staging sg{ctx, {}};
-    CopyBack back;
+    Staging sg(ctx);
     const lambda_film_query *dq;
     float *dout;
-    CK(sg.in(q, size_t(n), &dq), "stage queries");
-    CK(sg.out(out, size_t(n) * 4, &dout, back), "stage results");
+    sg.in(q, size_t(n), &dq);
+    sg.out(out, size_t(n) * 4, &dout);
+    CK(sg.begin(), "stage queries");
     lambda_status st = run_mlp<true>(ctx, dq, n, reinterpret_cast<float4 *>(dout));
     if (st != LAMBDA_OK) return st;
-    return finish_staging(ctx, back);
+    return sg.finish();
 }
 
 namespace {
@@ -1183,7 +1183,7 @@ extern "C" lambda_status lambda_surrogate_train(lambda_ctx *ctx, const lambda_tr
     // one allocation for the whole run, cut into 256-byte aligned parts, from the
     // context's staging memory where that keeps it: a cudaMalloc and its cudaFree take as
     // long as tens of training steps
-    Staging sg{ctx, {}};
+    Staging sg(ctx);
     void *arena = nullptr;
     const std::pair<DeviceBuffer *, size_t> parts[] = {
         {&x, size_t(N) * kRowStride * 4}, {&y, size_t(N) * 16}, {&ax, size_t(audit_n) * kRowStride * 4},
@@ -1191,7 +1191,8 @@ extern "C" lambda_status lambda_surrogate_train(lambda_ctx *ctx, const lambda_tr
         {&params, kParams * 4}, {&grad, size_t(slots) * kParams * 4}, {&m, kParams * 4}, {&v, kParams * 4}, {&loss, 64}};
     size_t arena_bytes = 0;
     for (const auto &q : parts) arena_bytes += (q.second + 255) / 256 * 256;
-    CK(sg.take(arena_bytes, &arena), "allocate training set");
+    sg.scratch(arena_bytes, &arena);
+    CK(sg.begin(), "allocate training set");
     size_t off = 0;
     for (const auto &q : parts) {
         *q.first = DeviceBuffer{static_cast<char *>(arena) + off, q.second};

@@ -95,3 +95,31 @@ print(json.dumps([first, left, second]))
     first, left, second = got
     assert first[2] == "" or "OUT_OF_MEMORY" in first[2]
     assert left == 0 and second[2] == ""
+
+
+@pytest.mark.parametrize("name", ["closest", "shadow", "film", "film_fp64"])
+def test_a_call_allocates_its_staging_once(on_cpu, name):
+    """The first call makes one allocation for all its arrays (and, for rays, the flags) and
+    frees none; calls that fit make none; a larger one replaces it. One that is larger than
+    the kept memory (64 MB) allocates once for itself."""
+    got = on_cpu(f'''
+call = calls["{name}"]
+small = [counted(lambda: call(n)) for n in (1000, 1000, 10)]
+grown = [counted(lambda: call(n)) for n in (20_000, 20_000, 1000)]
+large = [counted(lambda: call(n)) for n in (2_000_000, 2_000_000, 1000)]
+print(json.dumps([small, grown, large]))
+''')
+    small, grown, large = got
+    first = 2 if name in ("closest", "shadow") else 1
+    assert small == [[first, 0, ""], [0, 0, ""], [0, 0, ""]]
+    assert grown == [[1, 1, ""], [0, 0, ""], [0, 0, ""]]
+    assert large == [[1, 1, ""], [1, 1, ""], [0, 0, ""]]
+
+
+def test_a_large_call_takes_the_kept_memory_where_there_is_no_other(on_cpu):
+    got = on_cpu('''
+counted(lambda: calls["film"](1000))
+rt.fake_fail_malloc(1)
+print(json.dumps([counted(lambda: calls["film"](2_000_000)), rt.fake_pending(), counted(lambda: calls["film"](1000))]))
+''')
+    assert got == [[2, 2, ""], 0, [1, 0, ""]]
