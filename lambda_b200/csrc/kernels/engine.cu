@@ -1714,15 +1714,19 @@ cudaError_t Staging::begin() {
         if (e != cudaSuccess) return e;
         void *at = base + p.at;
         std::memcpy(p.dst, &at, sizeof(at));
-        if (p.src) e = cudaMemcpyAsync(at, p.src, p.bytes, cudaMemcpyHostToDevice, ctx->stream);
+        if (!p.src) continue;
+        e = cudaMemcpyAsync(at, p.src, p.bytes, cudaMemcpyHostToDevice, ctx->stream);
+        copying = true;
     }
     return e;
 }
 
 lambda_status Staging::finish() {
+    copying = true;
     for (const Part &p : parts)
         if (p.user) CK(cudaMemcpyAsync(p.user, base + p.at, p.bytes, cudaMemcpyDeviceToHost, ctx->stream), "copy results");
     CK(cudaStreamSynchronize(ctx->stream), "query");
+    copying = false;
     return LAMBDA_OK;
 }
 

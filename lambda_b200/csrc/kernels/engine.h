@@ -156,7 +156,10 @@ constexpr size_t kStagingKeep = size_t(64) << 20;
 class Staging {
 public:
     explicit Staging(lambda_ctx *c) : ctx(c) {}
+    // A call that ends early waits for its copies: a page-locked source is read behind the
+    // caller's back.
     ~Staging() {
+        if (copying) cudaStreamSynchronize(ctx->stream);
         if (own) cudaFree(own);
     }
     Staging(const Staging &) = delete;
@@ -194,4 +197,5 @@ private:
     size_t total = 0;
     char *base = nullptr;
     void *own = nullptr;
+    bool copying = false;
 };

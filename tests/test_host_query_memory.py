@@ -123,3 +123,19 @@ rt.fake_fail_malloc(1)
 print(json.dumps([counted(lambda: calls["film"](2_000_000)), rt.fake_pending(), counted(lambda: calls["film"](1000))]))
 ''')
     assert got == [[2, 2, ""], 0, [1, 0, ""]]
+
+
+@pytest.mark.parametrize("name", ["closest", "shadow", "film", "film_fp64"])
+def test_a_call_that_fails_waits_for_its_copies(on_cpu, name):
+    """A call whose launch fails returns only once the copies from the caller's arrays are
+    done: the caller may free page-locked arrays, which copy behind its back."""
+    got = on_cpu(f'''
+counted(lambda: calls["{name}"](1000))
+rt.fake_fail_launch(1)
+failed = counted(lambda: calls["{name}"](1000))
+waited = rt.fake_copies_waited_for()
+print(json.dumps([failed, waited, counted(lambda: calls["{name}"](1000))]))
+''')
+    failed, waited, after = got
+    assert "LAMBDA_ERR_CUDA" in failed[2] and after == [0, 0, ""]
+    assert waited == 1
