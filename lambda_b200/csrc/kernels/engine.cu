@@ -1635,8 +1635,9 @@ __global__ void __launch_bounds__(128) k_trace_closest(DeviceScene sc, const flo
     bool walking = false, overflow = false;
     for (;;) {
         if (k < 0) {
-            k = take_next(error + 1);
-            if (k >= n) break;
+            const unsigned idx = take_next(error + 1);
+            if (!lambda_host::item_left(idx, n)) break;
+            k = int(idx);
             const float *r = rays + 6 * size_t(k);
             wr = make_ray(mk(r[0], r[1], r[2]), mk(r[3], r[4], r[5]));
             if constexpr (!kQuantOf<L>) walking = flat_start(sc, wr, w);

@@ -25,6 +25,7 @@
 #include <cstdint>
 
 #include "dscene.cuh"
+#include "ray_counter.h"
 #include "tmm.cuh"
 
 namespace lambda_dev {
@@ -336,16 +337,16 @@ LAMBDA_KERNEL void __launch_bounds__(256, 4) k_intersect(int bounce, RenderParam
     }
 }
 
-// A traversal lane takes the next work index of its queue: the lanes that need one
-// take consecutive indices, one atomic per group.
-__device__ __forceinline__ int take_next(int *next) {
+// A traversal lane takes the next work index of its queue (ray_counter.h): the lanes
+// that need one take consecutive indices, one atomic per group.
+__device__ __forceinline__ unsigned take_next(int *next) {
     const int lane = threadIdx.x & 31;
     const unsigned need = __activemask();
     const int leader = __ffs(need) - 1;
     int base = 0;
     if (lane == leader) base = atomicAdd(next, __popc(need));
     base = __shfl_sync(need, base, leader);
-    return base + __popc(need & ((1u << lane) - 1u));
+    return lambda_host::taken_index(base, __popc(need & ((1u << lane) - 1u)));
 }
 
 // The end of path p's closest hit in the lane-by-lane kernel: store_hit, then its
@@ -394,8 +395,8 @@ LAMBDA_KERNEL void __launch_bounds__(256, 2) k_intersect_fetch(int bounce, Rende
         bool walking = false;
         for (;;) {
             if (p < 0) {
-                const int idx = take_next(next);
-                if (idx >= n) break;
+                const unsigned idx = take_next(next);
+                if (!lambda_host::item_left(idx, n)) break;
                 p = q[idx];
                 const float4 o4 = ps.ray_o[p], d4 = ps.ray_d[p];
                 wr = make_ray(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
@@ -414,8 +415,8 @@ LAMBDA_KERNEL void __launch_bounds__(256, 2) k_intersect_fetch(int bounce, Rende
         int best_obj = -1, best_inst = -1, inst = -1, sp = 0, ssp = 0;
         for (;;) {
             if (p < 0) {
-                const int idx = take_next(next);
-                if (idx >= n) break;
+                const unsigned idx = take_next(next);
+                if (!lambda_host::item_left(idx, n)) break;
                 p = q[idx];
                 const float4 o4 = ps.ray_o[p], d4 = ps.ray_d[p];
                 wr = make_ray(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
