@@ -600,16 +600,19 @@ __device__ __forceinline__ void train_mask(float (&v)[4][4], const float *act) {
 // half of the load pipe's cycles) and by the chain of barriers between its layers. Measured
 // per 8192-row step (B200, ncu): 31 us, against 167 us for one scalar output at a time
 // over unpadded rows; of those, one atomic per element on the epoch's loss took 38 us.
-// The epoch's loss is one FP32 running total. Each element is rounded to the precision
-// the total has about when its slice is added (the total before the minibatch and this
-// slice's share of it) before a warp adds its own up: adding the elements one by one
-// rounds them so, and the reported loss keeps its values.
+// The epoch's loss is one FP32 running total (*loss, which add_loss alone writes, after this
+// kernel). Each element is rounded to the precision the total has about when its slice is
+// added (the total before the minibatch and this slice's share of it) before a warp adds its
+// own up: adding the elements one by one rounds them so, and the reported loss keeps its
+// values. Each warp leaves its sum in a place of its own in loss_part ([gridDim.x][8]).
+constexpr int kLossParts = kTrainThreads / 32;
 __global__ void __launch_bounds__(kTrainThreads, 1) k_train_step(const float *params, const float *x, const float *y,
-                                                                int rows, float inv_count, float *partial, float *loss) {
+                                                                int rows, float inv_count, float *partial,
+                                                                const float *loss, float *loss_part) {
     extern __shared__ __align__(16) float ts[];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     float *grad = partial + size_t(blockIdx.x) * kParams;
-    const float before = *reinterpret_cast<volatile float *>(loss);  // the epoch's loss up to this minibatch
+    const float before = *loss;  // the epoch's loss up to this minibatch
     for (int e = tid; e < kH * kH; e += kTrainThreads) {
         const int o = e / kH, i = e % kH;
         const float w2 = bf16_round(params[oW2 + e]), w3 = bf16_round(params[oW3 + e]);
@@ -690,7 +693,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train_step(const float *pa
             float q = (total + sample_loss) - total;
 #pragma unroll
             for (int m = 16; m > 0; m >>= 1) q += __shfl_xor_sync(0xffffffffu, q, m);
-            if ((tid & 31) == 0) atomicAdd(loss, q);
+            if ((tid & 31) == 0) train_put(&loss_part[blockIdx.x * kLossParts + (tid >> 5)], q, first);
         }
         // output weights: one (output, feature) per thread; and the third layer's deltas
         {
@@ -797,14 +800,36 @@ __device__ __forceinline__ float sum_slots(const float *partial, int slots, int 
     return g;
 }
 
-__global__ void __launch_bounds__(256) k_grad_sum(const float *partial, int slots, int n, float *g) {
+// Adds the warps' parts of a minibatch's loss to the epoch's, in a fixed order: a block of
+// 256 threads.
+__device__ __forceinline__ void add_loss(const float *part, int n, float *loss) {
+    __shared__ float sums[8];
+    float a = 0.0f;
+    for (int k = threadIdx.x; k < n; k += 256) a += part[k];
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) a += __shfl_xor_sync(0xffffffffu, a, m);
+    if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = a;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 8; w++) a += sums[w];
+    *loss += a;
+}
+
+// The grids of k_grad_sum and k_adam: 32 parameters a block, and a last block for the loss.
+constexpr int kSumBlocks = (kParams + 31) / 32 + 1;
+
+__global__ void __launch_bounds__(256) k_grad_sum(const float *partial, int slots, int n, float *g,
+                                                  const float *loss_part, float *loss) {
+    if (blockIdx.x == gridDim.x - 1) return add_loss(loss_part, slots * kLossParts, loss);
     const int i = blockIdx.x * 32 + (threadIdx.x & 31);
     const float a = sum_slots(partial, slots, n, i);
     if (threadIdx.x < 32 && i < n) g[i] = a;
 }
 
 __global__ void __launch_bounds__(256) k_adam(float *p, const float *partial, int slots, float *m, float *v, int n, float lr,
-                                              float b1, float b2, float eps, float c1, float c2) {
+                                              float b1, float b2, float eps, float c1, float c2,
+                                              const float *loss_part, float *loss) {
+    if (blockIdx.x == gridDim.x - 1) return add_loss(loss_part, slots * kLossParts, loss);
     const int i = blockIdx.x * 32 + (threadIdx.x & 31);
     const float gi = sum_slots(partial, slots, n, i);
     if (threadIdx.x >= 32 || i >= n) return;
@@ -1178,7 +1203,7 @@ extern "C" lambda_status lambda_surrogate_train(lambda_ctx *ctx, const lambda_tr
     const Range rg = to_range(d.range);
     const int64_t N = d.samples;
     const int audit_n = 1 << 18;
-    DeviceBuffer x, y, ax, ay, params, grad, m, v, loss, aout, partial;
+    DeviceBuffer x, y, ax, ay, params, grad, m, v, loss, loss_part, aout, partial;
     const int slots = int(std::min<int64_t>(std::min<int64_t>(d.batch, N) / kTrainRows + 1, ctx->sm_count));
     // one allocation for the whole run, cut into 256-byte aligned parts, from the
     // context's staging memory where that keeps it: a cudaMalloc and its cudaFree take as
@@ -1188,7 +1213,8 @@ extern "C" lambda_status lambda_surrogate_train(lambda_ctx *ctx, const lambda_tr
     const std::pair<DeviceBuffer *, size_t> parts[] = {
         {&x, size_t(N) * kRowStride * 4}, {&y, size_t(N) * 16}, {&ax, size_t(audit_n) * kRowStride * 4},
         {&ay, size_t(audit_n) * 16}, {&aout, size_t(audit_n) * 16}, {&partial, 2 * kAuditBlocks * sizeof(double)},
-        {&params, kParams * 4}, {&grad, size_t(slots) * kParams * 4}, {&m, kParams * 4}, {&v, kParams * 4}, {&loss, 64}};
+        {&params, kParams * 4}, {&grad, size_t(slots) * kParams * 4}, {&m, kParams * 4}, {&v, kParams * 4}, {&loss, 64},
+        {&loss_part, size_t(slots) * kLossParts * 4}};
     size_t arena_bytes = 0;
     for (const auto &q : parts) arena_bytes += (q.second + 255) / 256 * 256;
     sg.scratch(arena_bytes, &arena);
@@ -1232,13 +1258,14 @@ extern "C" lambda_status lambda_surrogate_train(lambda_ctx *ctx, const lambda_tr
             k_train_step<<<blocks, kTrainThreads, kTrainSmem, st>>>(params.as<float>(), x.as<float>() + r0 * kRowStride,
                                                                    y.as<float>() + r0 * 4, rows,
                                                                    1.0f / float(rows * kOut), grad.as<float>(),
-                                                                   loss.as<float>());
+                                                                   loss.as<float>(), loss_part.as<float>());
             // cosine decay to 2% of the base rate
             const double frac = double(t) / double(std::max<int64_t>(1, total - 1));
             const float lr = float(d.learning_rate * (0.02 + 0.98 * 0.5 * (1 + std::cos(3.14159265358979 * frac))));
             const float c1 = float(1 - std::pow(0.9, double(t + 1))), c2 = float(1 - std::pow(0.999, double(t + 1)));
-            k_adam<<<(kParams + 31) / 32, 256, 0, st>>>(params.as<float>(), grad.as<float>(), blocks, m.as<float>(),
-                                                       v.as<float>(), kParams, lr, 0.9f, 0.999f, 1e-8f, c1, c2);
+            k_adam<<<kSumBlocks, 256, 0, st>>>(params.as<float>(), grad.as<float>(), blocks, m.as<float>(), v.as<float>(),
+                                               kParams, lr, 0.9f, 0.999f, 1e-8f, c1, c2, loss_part.as<float>(),
+                                               loss.as<float>());
         }
         CK(cudaGetLastError(), "launch training kernels");
         float h = 0;
@@ -1293,26 +1320,28 @@ extern "C" lambda_status lambda_surrogate_grad(lambda_ctx *ctx, const float *par
     for (int i = 0; i < n; i++)
         for (int k = 0; k < kIn; k++) rows[size_t(i) * kRowStride + k] = x[size_t(i) * kIn + k];
     const int slots = std::min((n + kTrainRows - 1) / kTrainRows, ctx->sm_count);
-    DeviceBuffer dp, dx, dy, dg, dl, partial;
+    DeviceBuffer dp, dx, dy, dg, dl, dlp, partial;
     CK(dp.upload(params, kParams * 4, ctx->stream), "stage");
     CK(dx.upload(rows.data(), rows.size() * 4, ctx->stream), "stage");
     CK(dy.upload(y, size_t(n) * 16, ctx->stream), "stage");
     CK(dg.reserve(kParams * 4), "stage");
     CK(dl.reserve(16), "stage");
+    CK(dlp.reserve(size_t(slots) * kLossParts * 4), "stage");
     CK(partial.reserve(size_t(slots) * kParams * 4), "stage");
     CK(cudaMemsetAsync(dl.ptr, 0, 16, ctx->stream), "stage");
     CK(cudaFuncSetAttribute(k_train_step, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem), "configure training kernel");
     k_train_step<<<slots, kTrainThreads, kTrainSmem, ctx->stream>>>(dp.as<float>(), dx.as<float>(), dy.as<float>(), n,
                                                                    1.0f / float(n * kOut), partial.as<float>(),
-                                                                   dl.as<float>());
-    k_grad_sum<<<(kParams + 31) / 32, 256, 0, ctx->stream>>>(partial.as<float>(), slots, kParams, dg.as<float>());
+                                                                   dl.as<float>(), dlp.as<float>());
+    k_grad_sum<<<kSumBlocks, 256, 0, ctx->stream>>>(partial.as<float>(), slots, kParams, dg.as<float>(), dlp.as<float>(),
+                                                    dl.as<float>());
     CK(cudaGetLastError(), "launch training kernel");
     CK(cudaMemcpyAsync(grad_out, dg.ptr, kParams * 4, cudaMemcpyDeviceToHost, ctx->stream), "read gradient");
     float l = 0;
     CK(cudaMemcpyAsync(&l, dl.ptr, 4, cudaMemcpyDeviceToHost, ctx->stream), "read loss");
     CK(cudaStreamSynchronize(ctx->stream), "gradient");
     if (loss_out) *loss_out = l;
-    for (DeviceBuffer *b : {&dp, &dx, &dy, &dg, &dl, &partial}) b->release();
+    for (DeviceBuffer *b : {&dp, &dx, &dy, &dg, &dl, &dlp, &partial}) b->release();
     return LAMBDA_OK;
 }
 
