@@ -690,7 +690,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train_step(const float *pa
             float slice = 0.0f;
             for (int w = 0; w < kTrainThreads / 32; w++) slice += ts[tLoss + w];
             const float total = before + slice * (float(r0 / kTrainRows) + 0.5f);
-            float q = (total + sample_loss) - total;
+            float q = isfinite(total) ? (total + sample_loss) - total : sample_loss;
 #pragma unroll
             for (int m = 16; m > 0; m >>= 1) q += __shfl_xor_sync(0xffffffffu, q, m);
             if ((tid & 31) == 0) train_put(&loss_part[blockIdx.x * kLossParts + (tid >> 5)], q, first);

@@ -108,3 +108,20 @@ def test_the_reported_loss_is_near_the_mean(ctx):
     want = float(np.mean((out - y.astype(np.float64)) ** 2))
     print(f"reported {rep.final_loss:.7g}, mean {want:.7g}: {rep.final_loss / want - 1:+.2%}")
     assert -5e-3 <= rep.final_loss / want - 1 <= 1e-3
+
+
+@pytest.mark.parametrize("n", [1, 64, 65, 10_000])
+@pytest.mark.parametrize("target", [1e25, -3e19, np.inf])
+def test_an_infinite_loss_stays_infinite(ctx, n, target):
+    """Squares beyond FP32 (or an infinite target) make the loss infinite, not NaN."""
+    rng = np.random.default_rng(2)
+    p = rng.normal(0, 0.3, N.MLP_PARAMS).astype(np.float32)
+    x = rng.uniform(-1, 1, (n, 5)).astype(np.float32)
+    y = rng.uniform(0, 1, (n, 4)).astype(np.float32)
+    y[n // 2, 1] = target
+    g = np.empty(N.MLP_PARAMS, np.float32)
+    loss = C.c_float()
+    st = ctx._lib.lambda_surrogate_grad(ctx._h, p.ctypes.data, x.ctypes.data, y.ctypes.data, n, g.ctypes.data,
+                                        C.byref(loss))
+    assert st == 0, ctx.last_error
+    assert loss.value == math.inf
