@@ -32,10 +32,7 @@ struct DeviceScene {
     const int *material_props;
     const float4 *scalar_tex;
     const int4 *spectrum_tex;
-    const int *light_inst;
-    const int *light_obj;
     const float *light_power;
-    const float *light_cdf;      // running sums of light_power in list order
     const float *material_emission;  // per material: average emission (0 if not emissive)
     const uint8_t *material_uv;      // per material: 1 if a texture it evaluates reads the hit's (u, v)
     const float4 *film_flat;         // per material: (n_outer, n_film, n_sub, 1) of a one-layer thin film whose
@@ -48,7 +45,7 @@ struct DeviceScene {
     // spheres 1080p, 16 spp 31.5 -> 30.7 ms.
     const float4 *tex_record;    // per spectrum texture: (kTex*, a, b, scale), see spectrum_texture4
     const float4 *film_layer;    // per material: the scalar texture of a one-layer thin film's thickness, else zeros
-    const float4 *light_record;  // per light: (light_cdf, light_power, instance and object bits)
+    const float4 *light_record;  // per light: (running sum of the powers in list order, power, instance and object bits)
     const uint32_t *instance_flags;  // bit 0: transform and inverse are exactly the identity; bit 1: also
                                      // alone in its TLAS leaf, whose box is its BLAS root's box
     const float4 *cie;           // [471] (x, y, z, 0) as float

@@ -550,10 +550,7 @@ extern "C" lambda_status lambda_scene_upload(lambda_ctx *ctx, const lambda_scene
     CK(b.material_props.upload(props.data(), props.size() * sizeof(int), s), "upload material properties");
     CK(b.scalar_tex.upload(stex.data(), stex.size() * sizeof(float4), s), "upload textures");
     CK(b.spectrum_tex.upload(sptex.data(), sptex.size() * sizeof(int4), s), "upload textures");
-    CK(b.light_inst.upload(d.light_instances, size_t(d.num_lights) * sizeof(int), s), "upload lights");
-    CK(b.light_obj.upload(d.light_objects, size_t(d.num_lights) * sizeof(int), s), "upload lights");
     CK(b.light_power.upload(d.light_powers, size_t(d.num_lights) * sizeof(float), s), "upload lights");
-    CK(b.light_cdf.upload(cdf.data(), cdf.size() * sizeof(float), s), "upload lights");
     CK(b.material_emission.upload(emission.data(), emission.size() * sizeof(float), s), "upload materials");
     CK(b.material_uv.upload(muv.data(), muv.size(), s), "upload materials");
     CK(b.film_flat.upload(film_flat.data(), film_flat.size() * sizeof(float4), s), "upload materials");
@@ -635,10 +632,7 @@ extern "C" lambda_status lambda_scene_upload(lambda_ctx *ctx, const lambda_scene
     ds.material_props = b.material_props.as<int>();
     ds.scalar_tex = b.scalar_tex.as<float4>();
     ds.spectrum_tex = b.spectrum_tex.as<int4>();
-    ds.light_inst = b.light_inst.as<int>();
-    ds.light_obj = b.light_obj.as<int>();
     ds.light_power = b.light_power.as<float>();
-    ds.light_cdf = b.light_cdf.as<float>();
     ds.material_emission = b.material_emission.as<float>();
     ds.material_uv = b.material_uv.as<uint8_t>();
     ds.film_flat = b.film_flat.as<float4>();
@@ -1007,9 +1001,9 @@ lambda_status render_pass(lambda_ctx *ctx, const lambda_job *jobs, const std::ve
     // path is in one material queue), so only the queue order depends on their
     // interleaving, and the next intersect waits for all three. The Lambertian
     // shade's shadow rays run on a stream of their own beside the next intersect:
-    // they add to the NEE radiance, which intersect no longer touches (it records a
-    // path's final emission apart), and the next Lambertian shade, which refills the
-    // NEE buffers, waits for them.
+    // they add to the NEE radiance, which intersect does not touch (a path's final
+    // emission is evaluated from its hit id when the sample is banked), and the next
+    // Lambertian shade, which refills the NEE buffers, waits for them.
     cudaError_t fork_err = cudaSuccess;
     auto wave = [&](StageProfiler *pr, cudaGraphConditionalHandle loop, int waves) -> int {
         int n = 0;

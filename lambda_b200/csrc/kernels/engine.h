@@ -56,7 +56,7 @@ struct HostBuffer {
 
 struct SceneBuffers {
     DeviceBuffer nodes, prims, tri, instances, spectra, spectrum_flat, cspectra, cspectrum_flat, materials,
-        material_props, scalar_tex, spectrum_tex, light_inst, light_obj, light_power, light_cdf, material_emission,
+        material_props, scalar_tex, spectrum_tex, light_power, material_emission,
         material_uv, film_flat, tex_record, film_layer, light_record,
         cie, perm, worley, instance_flags;
     DeviceBuffer wide[3], wide_leaves[3], wide_code[3];  // wide BVH of width 2, 4, 8
@@ -134,8 +134,8 @@ struct lambda_ctx {
         SceneBuffers &s = scene;
         RenderBuffers &r = rbuf;
         return {&s.nodes, &s.prims, &s.tri, &s.instances, &s.spectra, &s.spectrum_flat, &s.cspectra,
-                &s.cspectrum_flat, &s.materials, &s.material_props, &s.scalar_tex, &s.spectrum_tex, &s.light_inst,
-                &s.light_obj, &s.light_power, &s.light_cdf, &s.material_emission, &s.material_uv, &s.film_flat, &s.tex_record, &s.film_layer, &s.light_record, &s.cie, &s.perm, &s.worley, &s.instance_flags,
+                &s.cspectrum_flat, &s.materials, &s.material_props, &s.scalar_tex, &s.spectrum_tex,
+                &s.light_power, &s.material_emission, &s.material_uv, &s.film_flat, &s.tex_record, &s.film_layer, &s.light_record, &s.cie, &s.perm, &s.worley, &s.instance_flags,
                 &s.wide[0], &s.wide[1], &s.wide[2], &s.wide_leaves[0], &s.wide_leaves[1], &s.wide_leaves[2],
                 &s.wide_code[0], &s.wide_code[1], &s.wide_code[2], &s.wide_planes[0], &s.wide_planes[1], &s.wide_planes[2], &s.wide_q[0], &s.wide_q[1], &s.wide_q[2],
                 &r.rng, &r.film, &r.lam, &r.ray_o, &r.ray_d, &r.throughput, &r.radiance, &r.hit_id,
