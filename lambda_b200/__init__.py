@@ -430,15 +430,15 @@ def default_film_range() -> N.FilmRange:
 # structure-of-arrays words the stage must read and write (queue ids included),
 # not counting scene data, which is read-only and cache resident for small scenes.
 STAGE_BYTES = {
-    # film rw, radiance rw, lam rw, rng rw, hit id, ray/T w, queue (and the ray and T of a miss or an emitter hit)
-    "raygen": 16 * 2 + 16 * 2 + 16 * 2 + 8 * 2 + 16 + 16 * 3 + 4,
+    # film rw, radiance rw, lam rw, rng rw, the last sample's hit id, ray and T, the next one's ray/T w, queue
+    "raygen": 16 * 2 + 16 * 2 + 16 * 2 + 8 * 2 + 16 + 16 * 3 + 16 * 3 + 4,
     "intersect": 4 + 32 + 16 + 4,                          # queue id, ray read, hit id write, material push
     # the shade kernels rebuild the hit record from the ray and the hit id
     "shade_lambert": 4 + 32 + 16 + 16 * 2 + 8 * 2 + 32 + 16 + 64 + 8,  # queue, ray, hit id, T/lam, rng rw, ray w, T w, NEE w, pushes
     "shade_specular": 4 + 32 + 16 + 16 * 2 + 8 * 2 + 32 + 16 + 4,
     "shade_film": 4 + 32 + 16 + 16 * 2 + 8 * 2 + 32 + 16 + 4,
     "shadow": 4 + 16 * 3 + 8 + 16 * 2,                     # queue, NEE ray + weights, light ids, radiance rw
-    "finish": 16 * 3 + 12,
+    "finish": 16 * 3 + 16 + 16 * 3 + 12,                   # film, radiance, lam, the last hit id, ray and T, image w
     # surrogate thin film: queue, ray, hit id, T/lam, then 4 rows of 32 B and a domain flag
     "film_encode": 4 + 32 + 16 + 16 * 2 + 4 * 32 + 1,
     # queue, ray, hit id, T/lam, 4 outputs of 16 B, domain flag, rng rw, ray w, T w, push
