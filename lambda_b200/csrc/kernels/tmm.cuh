@@ -370,13 +370,14 @@ __device__ __forceinline__ double film_real_r(cx<double> r01, cx<double> r12, cx
 
 // Reflectances at one wavelength (k = 2 pi / lambda, thickness d) and, with want_t, the
 // transmittances. False past the decay at which the general product overflows its
-// exponentials' useful range.
+// exponentials' useful range, and past the growth (a negative thickness or wavelength) at
+// which the square of e here would: e^200 leaves it, and amplitudes up to 1e60, in range.
 __device__ __forceinline__ bool film_real_apply(const FilmReal &f, double d, double k, bool want_t, FilmResult<double> &out) {
     const double phase = 2.0 * (((f.n1 * k) * d) * f.c1);
     cx<double> e;
     double decay = 1.0;
     if (f.evanescent) {
-        if (!(fabs(phase) < 600.0)) return false;
+        if (!(phase > -200.0 && phase < 600.0)) return false;
         e = cx<double>{exp(-phase), 0.0};
         decay = e.re;
     } else {
