@@ -603,8 +603,9 @@ __device__ __forceinline__ void train_mask(float (&v)[4][4], const float *act) {
 // The epoch's loss is one FP32 running total (*loss, which add_loss alone writes, after this
 // kernel). Each element is rounded to the precision the total has about when its slice is
 // added (the total before the minibatch and this slice's share of it) before a warp adds its
-// own up: adding the elements one by one rounds them so, and the reported loss keeps its
-// values. Each warp leaves its sum in a place of its own in loss_part ([gridDim.x][8]).
+// own up: adding the elements one by one rounds them so, and the reported loss keeps the
+// values that runs have always reported (low, and lower the more samples an epoch has;
+// lambda_train_report says by how much). Each warp leaves its sum in a place of its own in loss_part ([gridDim.x][8]).
 constexpr int kLossParts = kTrainThreads / 32;
 __global__ void __launch_bounds__(kTrainThreads, 1) k_train_step(const float *params, const float *x, const float *y,
                                                                 int rows, float inv_count, float *partial,

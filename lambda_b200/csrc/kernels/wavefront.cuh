@@ -277,8 +277,8 @@ __device__ __forceinline__ int material_of(const DeviceScene &sc, int inst_mater
     return inst_material >= 0 ? inst_material : prim_material(load_prim(sc, obj));
 }
 
-// The emission used to be evaluated in the traversal kernels, which then spilled (64
-// registers, 336 B of spill loads); without it k_intersect runs the thin-film frame (B200,
+// The emission used to be evaluated in the traversal kernels, which then spilled more (64
+// registers, 204 B of spill loads at width 4, now 44); without it k_intersect runs the thin-film frame (B200,
 // 1080p, 16 spp) in 14.1 instead of 16.9 ms and the Cornell box's 144 launches in 2.6
 // instead of 3.1 ms, for 1.4 ms more in k_raygen on the former.
 // Stores path p's closest hit (best, obj, inst from the traversal, obj < 0 on a miss) and
