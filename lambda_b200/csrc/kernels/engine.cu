@@ -357,6 +357,9 @@ DeviceScene lambda_ctx::scene_view(int width) const {
     return v;
 }
 
+// A pass's statistics and, after them, its error flags: one clear and one copy back.
+constexpr size_t kPassStats = 8, kPassStatBytes = kPassStats * 8 + 16;
+
 namespace {
 
 // Child records (8 floats: min, code, max, 0) of every wide node to the plane form of
@@ -550,6 +553,10 @@ extern "C" lambda_status lambda_scene_upload(lambda_ctx *ctx, const lambda_scene
     CK(b.material_props.upload(props.data(), props.size() * sizeof(int), s), "upload material properties");
     CK(b.scalar_tex.upload(stex.data(), stex.size() * sizeof(float4), s), "upload textures");
     CK(b.spectrum_tex.upload(sptex.data(), sptex.size() * sizeof(int4), s), "upload textures");
+    // the fixed-size flags and counters of queries and passes lie among the scene's tables
+    CK(ctx->rbuf.error.reserve(16), "allocate flags");
+    CK(ctx->rbuf.wave.reserve(16), "allocate queues");
+    CK(ctx->rbuf.stats.reserve(kPassStatBytes), "allocate statistics");
     CK(b.light_power.upload(d.light_powers, size_t(d.num_lights) * sizeof(float), s), "upload lights");
     CK(b.material_emission.upload(emission.data(), emission.size() * sizeof(float), s), "upload materials");
     CK(b.material_uv.upload(muv.data(), muv.size(), s), "upload materials");
@@ -716,9 +723,6 @@ cudaError_t StageProfiler::collect() {
     used = 0;
     return cudaSuccess;
 }
-
-// A pass's statistics and, after them, its error flags: one clear and one copy back.
-constexpr size_t kPassStats = 8, kPassStatBytes = kPassStats * 8 + 16;
 
 lambda_status lambda_ctx::ensure_state(int pixels, int depth) {
     lambda_ctx *ctx = this;

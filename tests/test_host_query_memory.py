@@ -99,9 +99,9 @@ print(json.dumps([first, left, second]))
 
 @pytest.mark.parametrize("name", ["closest", "shadow", "film", "film_fp64"])
 def test_a_call_allocates_its_staging_once(on_cpu, name):
-    """The first call makes one allocation for all its arrays (and, for rays, the flags) and
-    frees none; calls that fit make none; a larger one replaces it. One that is larger than
-    the kept memory (64 MB) allocates once for itself."""
+    """The first call makes one allocation for all its arrays and frees none; calls that fit
+    make none; a larger one replaces it. One that is larger than the kept memory (64 MB)
+    allocates once for itself."""
     got = on_cpu(f'''
 call = calls["{name}"]
 small = [counted(lambda: call(n)) for n in (1000, 1000, 10)]
@@ -110,8 +110,7 @@ large = [counted(lambda: call(n)) for n in (2_000_000, 2_000_000, 1000)]
 print(json.dumps([small, grown, large]))
 ''')
     small, grown, large = got
-    first = 2 if name in ("closest", "shadow") else 1
-    assert small == [[first, 0, ""], [0, 0, ""], [0, 0, ""]]
+    assert small == [[1, 0, ""], [0, 0, ""], [0, 0, ""]]
     assert grown == [[1, 1, ""], [0, 0, ""], [0, 0, ""]]
     assert large == [[1, 1, ""], [1, 1, ""], [0, 0, ""]]
 
